@@ -145,6 +145,14 @@ __device__ __forceinline__ T warp_max(T x) {
   return x;
 }
 
+// A read-only word that no other warp of the SM will want (a run of columns
+// read once): it takes no L1 line from the values gathered beside it.
+__device__ __forceinline__ int ld_stream(const int *p) {
+  int v;
+  asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // Block-wide reduction; every thread of the block must call it.
 // smem needs 32 slots of T.
 template <typename T, bool IS_MAX = false>

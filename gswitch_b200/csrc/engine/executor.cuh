@@ -520,6 +520,12 @@ struct executor_t {
     // (pull_tm_k_of); other variants have no shape
     int shapes[2][2][8][2] = {};
   } tune;
+  int *dg_all_tile = nullptr;  // all-to-all pull: the vertex that owns each tile's first slot
+  int64_t all_tile_cap = 0;
+  // a run over one graph builds that table at its first level and keeps it
+  // until the run ends (all_tiles_keep); otherwise every level builds it
+  bool all_tiles_keep = false;
+  int all_tiles_built = 0;  // 1: over the out-edges, 2: over the in-edges
   twod_layout twod;                 // 2D-partition layout of the current graph
   int64_t persistent_levels = 0;    // levels run inside persistent launches
   int64_t persistent_launches = 0;  // persistent launches
@@ -540,6 +546,9 @@ struct executor_t {
     cudaFree(dg_hubs);
     dg_hubs = nullptr;
     hub_cap = 0;
+    cudaFree(dg_all_tile);
+    dg_all_tile = nullptr;
+    all_tile_cap = 0;
     if (h_psig) cudaFreeHost(h_psig);
     h_psig = d_psig = nullptr;
     for (auto &e : ev)
@@ -664,6 +673,37 @@ struct executor_t {
     tile_cap = need;
   }
 
+  // slots of the all-to-all pull: every in-edge and one per vertex
+  static int64_t all_tiles(int64_t n, int64_t arcs) { return (n + arcs + ALL_TILE - 1) / ALL_TILE; }
+  void ensure_all_tiles(int64_t n, int64_t arcs) {
+    const int64_t need = all_tiles(n, arcs) + 1;
+    if (need <= all_tile_cap) return;
+    cudaFree(dg_all_tile);
+    dg_all_tile = nullptr;
+    all_tile_cap = 0;
+    if (GSW_CUDA(cudaMalloc((void **)&dg_all_tile, sizeof(int) * need))) return;
+    all_tile_cap = need;
+  }
+
+  // the edge-balanced expands of a pattern that sends everything everywhere
+  template <bool PULL, typename E, typename F>
+  void launch_all(active_set_t &as, device_graph_t<CSR, E> &g, F &f, config_t &conf) {
+    using G = device_graph_t<CSR, E>;
+    const int64_t nt = all_tiles(as.size, g.nedges);
+    if (!(all_tiles_keep && all_tiles_built == (PULL ? 2 : 1))) {
+      ensure_all_tiles(as.size, g.nedges);
+      if (!ok()) return;
+      k_all_tiles<<<clamp_grid((nt + 255) / 256, sm_count() * 8), 256, 0, stream()>>>(
+          PULL ? g.dgr_row_off : g.dg_row_off, as.size, nt, dg_all_tile);
+      GSW_LAUNCHED();
+      all_tiles_built = PULL ? 2 : 1;
+    }
+    auto kern = PULL ? k_pull_all<G, F> : k_push_all<G, F>;
+    const int64_t want = (nt + ALL_WARPS - 1) / ALL_WARPS;
+    const int grid = opts().force_grid > 0 ? opts().force_grid : clamp_grid(want, resident_grid(kern, EXPAND_THREADS));
+    kern<<<grid, EXPAND_THREADS, 0, stream()>>>(as, g, f, conf, dg_all_tile, nt);
+  }
+
   template <bool PULL, int T, typename G>
   void strict_prepare(active_set_t &as, G &g, Status want) {
     const int64_t items = hints().frontier >= 0 ? hints().frontier : (as.fmt == Queue ? as.size + 1 : as.size);
@@ -771,6 +811,12 @@ struct executor_t {
           break;
         }
         case STRICT: {
+          // every vertex sends along all of its out-edges: no scan (the same
+          // line as for the pull below)
+          if (!fused && conf.conf_fromall && conf.conf_toall && !conf.conf_fixed && as.fmt == Bitmap) {
+            launch_all<false>(as, g, f, conf);
+            break;
+          }
           auto go = [&](auto tile) {
             constexpr int T = decltype(tile)::value;
             strict_prepare<false, T>(as, g, conf.want());
@@ -807,6 +853,15 @@ struct executor_t {
           // from-all pulls stage a per-vertex sum too: their tiles stop at
           // 1,024 slots (48 KB of static shared memory)
           const bool all = sizeof(typename F::wa_t) <= 4 && conf.conf_fromall;
+          if constexpr (sizeof(typename F::wa_t) <= 4) {
+            // every vertex gathers from all of its in-neighbours: no scan
+            // (a pattern with Fixed vertices drops out of levels, and a queue
+            // lists a subset, so both keep the scanned form below)
+            if (all && conf.conf_toall && !conf.conf_fixed && as.fmt == Bitmap) {
+              launch_all<true>(as, g, f, conf);
+              break;
+            }
+          }
           auto go = [&](auto tile) {
             constexpr int T = decltype(tile)::value;
             strict_prepare<true, T>(as, g, conf.want());

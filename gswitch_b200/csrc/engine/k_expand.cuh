@@ -925,6 +925,236 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_strict_all(active_set_t
 }
 
 // ===========================================================================
+// All-to-all expands: every vertex gathers from all of its in-neighbours, or
+// sends to all of its out-neighbours
+// ===========================================================================
+// Patterns whose every vertex both sends and receives at every level (from-all,
+// to-all, no Fixed vertices: PageRank) need no work list and no degree scan:
+// vertex v owns the slots off[v] + v .. off[v+1] + v (its in-edges, then one
+// slot that ends it), so a tile of ALL_TILE slots is a contiguous run of
+// columns and of vertices, both at most ALL_TILE long.  A warp takes a tile by
+// itself: no CTA barrier, and hubs cost one atomic per tile.
+// What bounds it: the L1 takes about one 128-byte line per cycle, so a warp's
+// gather of 32 unrelated values is 32 cycles; below that, the latency of column
+// load -> gather.  Lanes therefore read consecutive columns (the columns of a
+// hub are dense, so neighbouring lanes share lines), all ALL_PER gathers of a
+// lane are in flight before the first is used, and the values are turned in
+// shared memory so that each lane then sums ALL_PER consecutive edges serially;
+// only a lane's open end goes through a segmented shuffle scan.
+// PageRank level on RMAT 2^22 (128 M arcs): 520 us against 1,113 us for the
+// scanned form below it (one gather in flight per lane, a scan per 32 edges);
+// on a directed RMAT graph of 300,007 vertices (2.3 M arcs) 28 us.  A CTA-wide tile of 2,044 slots
+// measured 606 us (its warps wait for one another), 4, 6 and 8 CTAs per SM
+// 539, 577 and 656 us against 520 at 5 (more warps evict each other's lines).
+constexpr int ALL_PER = 8;
+constexpr int ALL_TILE = 32 * ALL_PER;
+constexpr int ALL_WARPS = EXPAND_THREADS / 32;
+
+// tile_lo[t] = the vertex that owns slot t * ALL_TILE: one thread per tile
+__global__ void __launch_bounds__(256) k_all_tiles(const int64_t *off, int64_t n, int64_t ntiles, int *tile_lo) {
+  for (int64_t t = threadIdx.x + (int64_t)blockIdx.x * blockDim.x; t < ntiles; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t s = t * ALL_TILE;
+    int64_t lo = 0, hi = n - 1;  // the smallest v whose end slot is at or past s
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (__ldg(off + mid + 1) + mid < s)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    tile_lo[t] = (int)lo;
+  }
+}
+
+template <typename G, typename F>
+__global__ void __launch_bounds__(EXPAND_THREADS, 5) k_pull_all(active_set_t as, G g, F f, config_t conf,
+                                                             const int *tile_lo, int64_t ntiles) {
+  using WA = typename F::wa_t;
+  // first edge of each vertex of the tile (from the tile's first); the values
+  // of the tile's edges, then the sums of its vertices.  A lane reads ALL_PER
+  // consecutive values: one pad word per ALL_PER keeps that free of conflicts.
+  __shared__ unsigned short s_begs[ALL_WARPS][ALL_TILE + 2];
+  __shared__ WA s_vals[ALL_WARPS][ALL_TILE + 32];
+  const int64_t n = as.size, m = g.nedges;
+  const Status want = conf.want();
+  const int lane = lane_id();
+  unsigned short *s_beg = s_begs[warp_id()];
+  WA *s_val = s_vals[warp_id()];
+  if (blockIdx.x == 0 && threadIdx.x == 0) account(as, conf, (unsigned long long)m);
+  const int64_t nwarps = (int64_t)gridDim.x * ALL_WARPS;
+  int64_t t = (int64_t)blockIdx.x * ALL_WARPS + warp_id();
+  if (t >= ntiles) return;
+  int lo = tile_lo[t], hi = t + 1 < ntiles ? tile_lo[t + 1] : (int)n - 1;
+  for (;;) {
+    const int64_t ea = t * ALL_TILE - lo;
+    const int64_t eb = t + 1 < ntiles ? (t + 1) * ALL_TILE - hi : m;
+    const int cnt = hi - lo + 1, ne = (int)(eb - ea);
+    int u[ALL_PER];
+    WA x[ALL_PER];
+#pragma unroll
+    for (int k = 0; k < ALL_PER; ++k) u[k] = 32 * k + lane < ne ? ld_stream(g.dgr_adj_list + ea + 32 * k + lane) : -1;
+    // the next tile's bounds and this tile's vertices arrive meanwhile
+    const int64_t tn = t + nwarps;
+    int nlo = 0, nhi = 0;
+    if (tn < ntiles) {
+      nlo = tile_lo[tn];
+      nhi = tn + 1 < ntiles ? tile_lo[tn + 1] : (int)n - 1;
+    }
+    for (int j = lane; j <= cnt; j += 32) {
+      const int64_t b = __ldg(g.dgr_row_off + lo + j) - ea;
+      s_beg[j] = (unsigned short)(b < 0 ? 0 : (b > ne ? ne : b));
+    }
+#pragma unroll
+    for (int k = 0; k < ALL_PER; ++k)
+      x[k] = u[k] >= 0 ? f.emit(u[k], g.fetch_edata_r(ea + 32 * k + lane), g) : f.data.zero;
+#pragma unroll
+    for (int k = 0; k < ALL_PER; ++k) {
+      const int e = 32 * k + lane;
+      s_val[e + e / ALL_PER] = x[k];
+    }
+    __syncwarp();
+    const int a = ALL_PER * lane, b = MIN(a + ALL_PER, ne);  // this lane's edges of the tile
+#pragma unroll
+    for (int k = 0; k < ALL_PER; ++k) x[k] = s_val[a + lane + k];
+    __syncwarp();  // s_val becomes the vertices' sums
+    int jfirst = -1, j = -1;  // the vertex of the first edge, of the open end
+    WA acc = f.data.zero, first = f.data.zero;
+    if (a < b) {
+      int l = 0, h = cnt;  // upper bound of a
+      while (l < h) {
+        const int mid = (l + h) >> 1;
+        if (s_beg[mid] <= a)
+          l = mid + 1;
+        else
+          h = mid;
+      }
+      jfirst = j = l - 1;
+      int end = s_beg[j + 1];
+#pragma unroll
+      for (int k = 0; k < ALL_PER; ++k) {
+        const int r = a + k;
+        if (r >= b) continue;
+        if (r >= end) {  // vertex j ends here; its first edges may lie in earlier lanes
+          if (j == jfirst)
+            first = acc;
+          else
+            s_val[j] = acc;
+          acc = f.data.zero;
+          end = s_beg[++j + 1];
+          if (r >= end) {  // past vertices without edges, of which a skewed graph has long runs
+            l = j + 1, h = cnt;
+            while (l < h) {
+              const int mid = (l + h) >> 1;
+              if (s_beg[mid] <= r)
+                l = mid + 1;
+              else
+                h = mid;
+            }
+            j = l - 1;
+            end = s_beg[j + 1];
+          }
+        }
+        f.comp(&acc, x[k], g);
+      }
+    }
+    // open ends: runs of lanes with the same vertex, summed toward their last
+    // lane, or into the lane that closes the vertex
+    const int pj = __shfl_up_sync(FULL, j, 1);
+    const unsigned starts = __ballot_sync(FULL, lane == 0 || pj != j);
+    const int head = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const WA ox = shfl_up_any(acc, d);
+      if (lane - d >= head) f.comp(&acc, ox, g);
+    }
+    const WA before = shfl_up_any(acc, 1);
+    const int nj = __shfl_down_sync(FULL, jfirst, 1);
+    if (jfirst != j) {
+      if (lane > 0 && pj == jfirst) f.comp(&first, before, g);
+      s_val[jfirst] = first;
+    }
+    if (j >= 0 && (lane == 31 || nj != j)) s_val[j] = acc;
+    __syncwarp();
+    for (int i = lane; i < cnt; i += 32) {
+      if (s_beg[i + 1] == s_beg[i]) continue;  // no edge of this vertex in the tile
+      const int v = lo + i;
+      if (as.fetch_bitmap(v, want) < 0) continue;
+      // only the tile's first and last vertex can continue in another tile
+      const bool whole = (i > 0 || __ldg(g.dgr_row_off + v) >= ea) && (i + 1 < cnt || __ldg(g.dgr_row_off + v + 1) <= eb);
+      if (whole)
+        f.comp(f.wa_of(v), s_val[i], g);
+      else
+        f.compAtomic(f.wa_of(v), s_val[i], g);
+    }
+    if (tn >= ntiles) break;
+    t = tn;
+    lo = nlo;
+    hi = nhi;
+    __syncwarp();
+  }
+}
+
+// The push over the same tiles (of the out-edges).  Its atomics bound it, one
+// per arc and all of a hub's at one address; the tiles spare it the degree scan
+// (three launches a level) and the per-edge search.  Lanes work on consecutive
+// edges, whose targets share sectors: with ALL_PER consecutive edges to a lane,
+// as in the pull, RMAT 2^22 took 1,932 us a level.  PageRank level against the
+// scanned push: directed RMAT of 300,007 vertices 79 -> 62 us, RMAT 2^22
+// 1,676 -> 1,572 us.
+template <typename G, typename F>
+__global__ void __launch_bounds__(EXPAND_THREADS) k_push_all(active_set_t as, G g, F f, config_t conf,
+                                                             const int *tile_lo, int64_t ntiles) {
+  __shared__ unsigned short s_begs[ALL_WARPS][ALL_TILE + 2];
+  __shared__ unsigned short s_owns[ALL_WARPS][ALL_TILE + 32];  // the tile's vertex that owns each edge
+  const int64_t n = as.size, m = g.nedges;
+  const Status want = conf.want();
+  const int lane = lane_id();
+  unsigned short *s_beg = s_begs[warp_id()], *s_own = s_owns[warp_id()];
+  if (blockIdx.x == 0 && threadIdx.x == 0) account(as, conf, (unsigned long long)m);
+  const int64_t nwarps = (int64_t)gridDim.x * ALL_WARPS;
+  for (int64_t t = (int64_t)blockIdx.x * ALL_WARPS + warp_id(); t < ntiles; t += nwarps) {
+    const int lo = tile_lo[t], hi = t + 1 < ntiles ? tile_lo[t + 1] : (int)n - 1;
+    const int64_t ea = t * ALL_TILE - lo;
+    const int64_t eb = t + 1 < ntiles ? (t + 1) * ALL_TILE - hi : m;
+    const int cnt = hi - lo + 1, ne = (int)(eb - ea);
+    int u[ALL_PER];
+#pragma unroll
+    for (int k = 0; k < ALL_PER; ++k) u[k] = 32 * k + lane < ne ? ld_stream(g.dg_adj_list + ea + 32 * k + lane) : -1;
+    __syncwarp();  // the previous tile has been read
+    for (int j = lane; j <= cnt; j += 32) {
+      const int64_t b = __ldg(g.dg_row_off + lo + j) - ea;
+      s_beg[j] = (unsigned short)(b < 0 ? 0 : (b > ne ? ne : b));
+    }
+    __syncwarp();
+    const int a = ALL_PER * lane, b = MIN(a + ALL_PER, ne);
+    int j = -1, end = 0;
+    for (int r = a; r < b; ++r) {
+      if (r >= end) {
+        int l = j + 1, h = cnt;
+        while (l < h) {
+          const int mid = (l + h) >> 1;
+          if (s_beg[mid] <= r)
+            l = mid + 1;
+          else
+            h = mid;
+        }
+        j = l - 1;
+        end = s_beg[j + 1];
+      }
+      s_own[r + lane] = (unsigned short)j;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < ALL_PER; ++k) {
+      if (u[k] < 0) continue;
+      const int e = 32 * k + lane;
+      const int v = lo + s_own[e + e / ALL_PER];
+      if (as.fetch_bitmap(v, want) >= 0) f.compAtomic(f.wa_of(u[k]), f.emit(v, g.fetch_edata(ea + e), g), g);
+    }
+  }
+}
+
+// ===========================================================================
 // Hub runs: the edges [a, a + len) of one vertex swept by the whole CTA
 // ===========================================================================
 // How a CTA reads a hub's columns (config_t::conf_hub_path):

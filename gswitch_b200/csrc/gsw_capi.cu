@@ -2245,6 +2245,8 @@ gsw_status gsw_pagerank(gsw_ctx *ctx, gsw_graph *gr, const gsw_run_opts *o, floa
                               dl_key() << f.data.dg_wa << f.data.dg_ra << f.damp << f.eps << f.data.zero, as, g, f,
                               conf, fets, op->max_iters, MAX_LEVELS, op->selector))
     return eg.finish();
+  executor.all_tiles_keep = !captured;  // one graph for the whole run
+  executor.all_tiles_built = 0;
   timer tm(ctx);
   int steps = 0;
   if (captured) dl_launch(R);
@@ -2262,6 +2264,7 @@ gsw_status gsw_pagerank(gsw_ctx *ctx, gsw_graph *gr, const gsw_run_opts *o, floa
     steps++;
     if (finish(as, g, f, conf)) break;
   }
+  executor.all_tiles_keep = false;
   const double ms = tm.stop();
   if (captured) {
     gsw_run_stats tmp;
