@@ -7,6 +7,7 @@
 // drive inspector / selector / executor (file:line per runner).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <map>
 #include <unordered_map>
@@ -21,6 +22,7 @@
 #include "engine/mlp.cuh"
 #include "graphgen.cuh"
 #include "bc_batch.cuh"
+#include "gc_dag.cuh"
 #include "mbfs.cuh"
 
 using namespace gsw;
@@ -40,6 +42,7 @@ struct gsw_graph {
   int64_t ncoo = -1;
   double attr[6] = {0, 0, 0, 0, 0, 0};
   double mean_weight = 0;
+  int rows_sorted = -1;   // every adjacency ascends (-1: not looked at yet)
   std::vector<int> hdeg;  // host copy of the out-degrees (root features, roots)
   struct twod_store {
     uint64_t *edge = nullptr;
@@ -2539,10 +2542,81 @@ gsw_status gsw_bc(gsw_ctx *ctx, gsw_graph *gr, int32_t root, const gsw_run_opts 
 // ---------------------------------------------------------------------------
 // GC: application/gc.cu:76-99 (loop) and :101-122 (set-up)
 // ---------------------------------------------------------------------------
+// Nothing about the level loop is asked for: no forced choice, no per-level
+// record, no captured or per-launch form.
+static bool unforced(const gsw_run_opts *o) {
+  return !record_sink() && !g_label &&
+         (!o || (o->direction < 0 && o->asfmt < 0 && o->lb < 0 && o->fusion < 0 && !o->verbose && !o->timing &&
+                 o->expand_grid == 0 && !o->account && o->persistent != 0 && !o->barrier_test && !o->captured));
+}
+
+static bool rows_sorted(gsw_graph *g) {
+  if (g->rows_sorted < 0) {
+    long long *d = (long long *)g->ctx->buf("row_descents", sizeof(long long)), h = 1;
+    if (!d) return false;
+    GSW_CUDA(cudaMemsetAsync(d, 0, sizeof(long long), stream()));
+    k_row_descents<<<grid_for(g->m), 256, 0, stream()>>>(g->off, g->col, g->n, g->m, d);
+    GSW_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, stream()));
+    GSW_CUDA(cudaStreamSynchronize(stream()));
+    if (!ok()) return false;
+    g->rows_sorted = h == 0;
+  }
+  return g->rows_sorted == 1;
+}
+
+// the colouring in dependency order (gc_dag.cuh): the level loop's colours
+static gsw_status gc_dag_run(gsw_ctx *ctx, gsw_graph *gr, int32_t *colors, gsw_run_stats *st, entry_guard &eg) {
+  const size_t row = sizeof(int) * (gr->n + 1);
+  int *wait = (int *)ctx->buf("wa", row), *colour = (int *)ctx->buf("ra", row), *low = (int *)ctx->buf("gc_low", row);
+  int *q0 = (int *)ctx->buf("gc_q0", row), *q1 = (int *)ctx->buf("gc_q1", row);
+  gc_state_t *S = (gc_state_t *)ctx->buf("gc_state", sizeof(gc_state_t));
+  if (!wait || !colour || !low || !q0 || !q1 || !S) return eg.finish();
+  auto g = gr->view<Empty>();
+  unsigned long long budget = 2000000000ull;  // per barrier wait
+  // one warp per 32 vertices fills the grid; a small graph takes fewer CTAs
+  const int grid = clamp_grid((gr->n + GC_THREADS - 1) / GC_THREADS, resident_grid(k_gc_dag, GC_THREADS));
+  gc_state_t h{};
+  GSW_CUDA(cudaMemsetAsync(S, 0, sizeof(gc_state_t), stream()));
+  timer tm(ctx);
+  for (int first = 1; ok(); first = 0) {
+    if (!first) GSW_CUDA(cudaMemsetAsync(S, 0, offsetof(gc_state_t, pub), stream()));
+    void *args[] = {(void *)&g,  (void *)&wait, (void *)&low, (void *)&colour, (void *)&q0,
+                    (void *)&q1, (void *)&S,    (void *)&first, (void *)&budget};
+    if (GSW_CUDA(cudaLaunchCooperativeKernel((const void *)k_gc_dag, grid, GC_THREADS, args, 0, stream()))) break;
+    GSW_LAUNCHED();
+    GSW_CUDA(cudaMemcpyAsync(&h, S, sizeof(h), cudaMemcpyDeviceToHost, stream()));
+    GSW_CUDA(cudaStreamSynchronize(stream()));
+    if (h.status == 2) set_error(GSW_ERR_TIMEOUT, "%s", "colouring: grid barrier timed out");
+    if (h.status != 1) break;
+  }
+  const double ms = tm.stop();
+  // a vertex that is its own neighbour waits for itself, as in the level loop
+  if (ok() && (int64_t)h.coloured != gr->n)
+    set_error(GSW_ERR_TIMEOUT, "%s", "level loop did not converge within the level cap");
+  if (st) {
+    st->ms = ms;
+    st->levels = h.at.level;
+    st->edges = gr->m / 2;
+    st->launches = launch_count();
+    // one persistent launch: push, queue, its own mapping (warp)
+    st->level_cfg[0] = ((int)WM << 2) | (1 << 5) | (1 << 6);
+    st->level_frontier[0] = -1;
+    st->level_ms[0] = st->level_inspect_ms[0] = 0;
+    st->level_edges[0] = 0;
+    st->ntrace = 1;
+  }
+  if (colors && ok())
+    GSW_CUDA(cudaMemcpyAsync(colors, colour, sizeof(int) * gr->n, cudaMemcpyDeviceToHost, stream()));
+  GSW_CUDA(cudaStreamSynchronize(stream()));
+  return eg.finish();
+}
+
 gsw_status gsw_gc(gsw_ctx *ctx, gsw_graph *gr, const gsw_run_opts *o, int32_t *colors, gsw_run_stats *st) {
   entry_guard eg(ctx);
   if (!ctx || !gr) return fail(GSW_ERR_INVALID_ARG, "gsw_gc: bad arguments");
   begin_stats(st);
+  if (unforced(o) && rows_sorted(gr)) return gc_dag_run(ctx, gr, colors, st, eg);
+  if (!ok()) return eg.finish();
   auto g = gr->view<Empty>();
   app::GC f;
   f.data.size = gr->n;
