@@ -22,6 +22,7 @@
 #include "engine/mlp.cuh"
 #include "graphgen.cuh"
 #include "bc_batch.cuh"
+#include "cc_forest.cuh"
 #include "gc_dag.cuh"
 #include "mbfs.cuh"
 
@@ -42,6 +43,8 @@ struct gsw_graph {
   int64_t ncoo = -1;
   double attr[6] = {0, 0, 0, 0, 0, 0};
   double mean_weight = 0;
+  int both_ends = -1;     // every arc is listed from both ends (-1: not looked at yet)
+  int64_t up_arcs = -1;   // arcs v -> u with u > v, counted with it
   int rows_sorted = -1;   // every adjacency ascends (-1: not looked at yet)
   std::vector<int> hdeg;  // host copy of the out-degrees (root features, roots)
   struct twod_store {
@@ -2110,10 +2113,86 @@ static bool cc_captured_run(gsw_ctx *ctx, device_graph_t<COO, Empty> g, app::CC 
   return ok();
 }
 
+// Nothing about the level loop is asked for: no forced choice, no per-level
+// record, no captured or per-launch form.
+static bool unforced(const gsw_run_opts *o) {
+  return !record_sink() && !g_label &&
+         (!o || (o->direction < 0 && o->asfmt < 0 && o->lb < 0 && o->fusion < 0 && !o->verbose && !o->timing &&
+                 o->expand_grid == 0 && !o->account && o->persistent != 0 && !o->barrier_test && !o->captured));
+}
+
+// is the graph stored with every arc listed from both ends? (an undirected
+// upload that lists each edge once is taken as it is by the edge-centric loop)
+static bool both_ends(gsw_ctx *ctx, gsw_graph *g) {
+  if (g->both_ends < 0) {
+    executor_t &ex = ctx->executor;
+    cc_state_t *S = (cc_state_t *)ctx->buf("cc_state", sizeof(cc_state_t)), h{};
+    ex.ensure_all_tiles(g->n, g->m);
+    if (!S || !ok()) return false;
+    const int64_t nt = executor_t::all_tiles(g->n, g->m);
+    GSW_CUDA(cudaMemsetAsync(S, 0, sizeof(cc_state_t), stream()));
+    k_all_tiles<<<clamp_grid((nt + 255) / 256, sm_count() * 8), 256, 0, stream()>>>(g->off, g->n, nt, ex.dg_all_tile);
+    k_arc_pairs<<<clamp_grid((nt + ALL_WARPS - 1) / ALL_WARPS, resident_grid(k_arc_pairs, EXPAND_THREADS)),
+                  EXPAND_THREADS, 0, stream()>>>(g->off, g->col, g->n, g->m, ex.dg_all_tile, nt, S);
+    GSW_LAUNCHED();
+    GSW_CUDA(cudaMemcpyAsync(&h, S, sizeof(h), cudaMemcpyDeviceToHost, stream()));
+    GSW_CUDA(cudaStreamSynchronize(stream()));
+    if (!ok()) return false;
+    g->both_ends = h.balance == 0;
+    g->up_arcs = (int64_t)h.up;
+  }
+  return g->both_ends == 1;
+}
+
+// components by sampled hooking (cc_forest.cuh): the loop's labels
+static gsw_status cc_forest_run(gsw_ctx *ctx, gsw_graph *gr, int32_t *labels, gsw_run_stats *st, entry_guard &eg) {
+  const int64_t n = gr->n;
+  int *comp = (int *)ctx->buf("wa", sizeof(int) * (n + 1));
+  cc_state_t *S = (cc_state_t *)ctx->buf("cc_state", sizeof(cc_state_t));
+  cc_piece_t *piece = (cc_piece_t *)ctx->buf("cc_pieces", sizeof(cc_piece_t) * (gr->m / (CC_ROW_PIECE / 2) + 2));
+  if (!comp || !S || !piece) return eg.finish();
+  const int grid = clamp_grid((n + CC_THREADS - 1) / CC_THREADS, sm_count() * 8);
+  timer tm(ctx);
+  k_cc_start<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp);
+  GSW_LAUNCHED();
+  for (int last = 0; last < 2; ++last) {
+    k_cc_link_one<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp, last != 0);
+    GSW_LAUNCHED();
+  }
+  k_cc_flatten<<<grid, CC_THREADS, 0, stream()>>>(comp, n);
+  GSW_LAUNCHED();
+  k_cc_common<<<1, CC_SAMPLE, 0, stream()>>>(comp, n, S);
+  GSW_LAUNCHED();
+  k_cc_rest<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp, S, piece);
+  GSW_LAUNCHED();
+  k_cc_pieces<<<sm_count() * 8, CC_THREADS, 0, stream()>>>(gr->col, comp, S, piece);
+  GSW_LAUNCHED();
+  k_cc_flatten<<<grid, CC_THREADS, 0, stream()>>>(comp, n);
+  GSW_LAUNCHED();
+  const double ms = tm.stop();
+  if (st) {
+    st->ms = ms;
+    st->levels = 1;
+    st->edges = gr->up_arcs;
+    st->launches = launch_count();
+    st->level_cfg[0] = (1 << 1) | ((int)WM << 2);  // one pass, bitmap form, as the loop's first level
+    st->level_frontier[0] = gr->up_arcs;
+    st->level_ms[0] = st->level_inspect_ms[0] = 0;
+    st->level_edges[0] = 0;
+    st->ntrace = 1;
+  }
+  if (labels && ok()) GSW_CUDA(cudaMemcpyAsync(labels, comp, sizeof(int) * n, cudaMemcpyDeviceToHost, stream()));
+  GSW_CUDA(cudaStreamSynchronize(stream()));
+  return eg.finish();
+}
+
 gsw_status gsw_cc(gsw_ctx *ctx, gsw_graph *gr, const gsw_run_opts *o, int32_t *labels, gsw_run_stats *st) {
   entry_guard eg(ctx);
   if (!ctx || !gr) return fail(GSW_ERR_INVALID_ARG, "gsw_cc: bad arguments");
   begin_stats(st);
+  if (unforced(o) && !gr->directed && gr->m > 0 && both_ends(ctx, gr) && gr->up_arcs > 0)
+    return cc_forest_run(ctx, gr, labels, st, eg);
+  if (!ok()) return eg.finish();
   if (ensure_coo(gr)) return eg.finish();
   device_graph_t<COO, Empty> g;
   g.dg_coo = gr->coo;
@@ -2542,14 +2621,6 @@ gsw_status gsw_bc(gsw_ctx *ctx, gsw_graph *gr, int32_t root, const gsw_run_opts 
 // ---------------------------------------------------------------------------
 // GC: application/gc.cu:76-99 (loop) and :101-122 (set-up)
 // ---------------------------------------------------------------------------
-// Nothing about the level loop is asked for: no forced choice, no per-level
-// record, no captured or per-launch form.
-static bool unforced(const gsw_run_opts *o) {
-  return !record_sink() && !g_label &&
-         (!o || (o->direction < 0 && o->asfmt < 0 && o->lb < 0 && o->fusion < 0 && !o->verbose && !o->timing &&
-                 o->expand_grid == 0 && !o->account && o->persistent != 0 && !o->barrier_test && !o->captured));
-}
-
 static bool rows_sorted(gsw_graph *g) {
   if (g->rows_sorted < 0) {
     long long *d = (long long *)g->ctx->buf("row_descents", sizeof(long long)), h = 1;
