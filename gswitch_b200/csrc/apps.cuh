@@ -58,6 +58,8 @@ struct SSSP : Functor<VC, int, int, int> {
     return old > nv ? data.win().in((float)nv) : false;
   }
   __device__ __forceinline__ bool cond(int v, int msg, GW) { return *wa_of(v) > msg; }
+  // distances only fall, so one that is no larger now drops the message for good
+  __device__ __forceinline__ bool drops(int v, int msg, GW) { return *wa_of(v) <= msg; }
   __device__ __forceinline__ bool exit(int v, GW) { return *wa_of(v) != *ra_of(v); }
 };
 

@@ -226,6 +226,10 @@ struct Functor<VC, WA, RA, E> {
   __device__ bool cond(int, WA, G) { return false; }
   __device__ bool comp(WA *, WA, G) { return true; }
   __device__ bool compAtomic(WA *, WA, G) { return true; }
+  // engine extension: may say true only where compAtomic would return false and
+  // change nothing, from a value that may be older than the current one; a push
+  // then spares the atomic
+  __device__ bool drops(int, WA, G) { return false; }
   __device__ bool exit(int, G) { return false; }
 };
 

@@ -45,7 +45,7 @@ __device__ __forceinline__ void push_edge_std(active_set_t &as, const G &g, F &f
   if (tp && !conf.conf_toall) tp = as.bitmap.is_inactive(u);
   if (tp) {
     auto vd = f.emit(v, g.fetch_edata(ei), g);
-    f.compAtomic(f.wa_of(u), vd, g);
+    if (!f.drops(u, vd, g)) f.compAtomic(f.wa_of(u), vd, g);
   }
 }
 
@@ -55,9 +55,57 @@ __device__ __forceinline__ bool push_edge_fused(active_set_t &as, const G &g, F 
   auto vd = f.emit(v, g.fetch_edata(ei), g);
   bool tp = true;
   if (!conf.conf_toall) tp = f.cond(u, vd, g);
-  if (tp) tp = f.compAtomic(f.wa_of(u), vd, g);
+  if (tp) tp = !f.drops(u, vd, g) && f.compAtomic(f.wa_of(u), vd, g);
   if (tp) tp = as.bitmap.mark_duplicate_atomic(u);
   return tp;
+}
+
+// The same for EDGE_BATCH edges of a thread (u < 0: none), step by step over
+// all of them.  An edge is a chain of dependent accesses (column, message's
+// parts, target's state, atomics); one at a time, a level waits for each chain
+// in turn.  With the messages that a target's present value already drops left
+// out before their atomic, the two large edge-balanced levels of SSSP on RMAT
+// 2^22 went from 1,037 and 1,569 us to 678 and 870.  tp: the edges whose target
+// a fused level appends.
+constexpr int EDGE_BATCH = 4;
+template <bool FUSED, typename G, typename F>
+__device__ __forceinline__ void push_edges(active_set_t &as, const G &g, F &f, const config_t &conf,
+                                           const int (&v)[EDGE_BATCH], const int (&u)[EDGE_BATCH],
+                                           const int64_t (&ei)[EDGE_BATCH], bool (&tp)[EDGE_BATCH]) {
+  typename F::wa_t msg[EDGE_BATCH];
+#pragma unroll
+  for (int k = 0; k < EDGE_BATCH; ++k) tp[k] = u[k] >= 0;
+  if (!FUSED && conf.conf_pruning) {
+    uint32_t seen[EDGE_BATCH];
+#pragma unroll
+    for (int k = 0; k < EDGE_BATCH; ++k) seen[k] = tp[k] ? as.bitmap.visited.load_word(u[k]) : 0;
+#pragma unroll
+    for (int k = 0; k < EDGE_BATCH; ++k) {
+      if (!tp[k]) continue;
+      const uint32_t m = 1u << (u[k] & 31);
+      tp[k] = !(seen[k] & m);
+      if (tp[k]) atomicOr(as.bitmap.visited.dg_bits + (u[k] >> 5), m);
+    }
+  }
+  if (!FUSED && !conf.conf_toall) {
+#pragma unroll
+    for (int k = 0; k < EDGE_BATCH; ++k) tp[k] = tp[k] && as.bitmap.is_inactive(u[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < EDGE_BATCH; ++k)
+    if (tp[k]) msg[k] = f.emit(v[k], g.fetch_edata(ei[k]), g);
+  if (FUSED && !conf.conf_toall) {
+#pragma unroll
+    for (int k = 0; k < EDGE_BATCH; ++k) tp[k] = tp[k] && f.cond(u[k], msg[k], g);
+  }
+#pragma unroll
+  for (int k = 0; k < EDGE_BATCH; ++k) tp[k] = tp[k] && !f.drops(u[k], msg[k], g);
+#pragma unroll
+  for (int k = 0; k < EDGE_BATCH; ++k) tp[k] = tp[k] && f.compAtomic(f.wa_of(u[k]), msg[k], g);
+  if (FUSED) {
+#pragma unroll
+    for (int k = 0; k < EDGE_BATCH; ++k) tp[k] = tp[k] && as.bitmap.mark_duplicate_atomic(u[k]);
+  }
 }
 
 // Fused levels append the vertices they activate to the output queue.  A warp
@@ -365,20 +413,26 @@ __device__ __forceinline__ void push_wm_body(active_set_t &as, const G &g, F &f,
     s_v[w][lane] = v;
     s_st[w][lane] = st;
     __syncwarp();
-    for (int base = 0; base < total; base += 32) {
-      const int i = base + lane;
-      bool tp = false;
-      int u = -1;
-      if (i < total) {
-        const int id = upper_bound(s_scan[w], 32, i) - 1;
-        const int64_t ei = s_st[w][id] + (i - s_scan[w][id]);
-        u = __ldg(g.dg_adj_list + ei);
-        if (FUSED)
-          tp = push_edge_fused(as, g, f, conf, s_v[w][id], u, ei);
-        else
-          push_edge_std(as, g, f, conf, s_v[w][id], u, ei);
+    for (int base = 0; base < total; base += 32 * EDGE_BATCH) {
+      int ev[EDGE_BATCH], u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool tp[EDGE_BATCH];
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int i = base + 32 * k + lane;
+        ev[k] = u[k] = -1;
+        ei[k] = 0;
+        if (i < total) {
+          const int id = upper_bound(s_scan[w], 32, i) - 1;
+          ev[k] = s_v[w][id];
+          ei[k] = s_st[w][id] + (i - s_scan[w][id]);
+          u[k] = __ldg(g.dg_adj_list + ei[k]);
+        }
       }
-      if (FUSED) stage.push(tp, u);
+      push_edges<FUSED>(as, g, f, conf, ev, u, ei, tp);
+      if (FUSED)
+#pragma unroll
+        for (int k = 0; k < EDGE_BATCH; ++k) stage.push(tp[k], u[k]);
     }
     __syncwarp();
   }
@@ -486,20 +540,26 @@ __device__ __forceinline__ void push_cm_body(active_set_t &as, const G &g, F &f,
     s_v[threadIdx.x] = v;
     s_st[threadIdx.x] = st;
     __syncthreads();
-    for (int base = 0; base < total; base += B) {
-      const int i = base + threadIdx.x;
-      bool tp = false;
-      int u = -1;
-      if (i < total) {
-        const int id = upper_bound(s_scan, B, i) - 1;
-        const int64_t ei = s_st[id] + (i - s_scan[id]);
-        u = __ldg(g.dg_adj_list + ei);
-        if (FUSED)
-          tp = push_edge_fused(as, g, f, conf, s_v[id], u, ei);
-        else
-          push_edge_std(as, g, f, conf, s_v[id], u, ei);
+    for (int base = 0; base < total; base += B * EDGE_BATCH) {
+      int ev[EDGE_BATCH], u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool tp[EDGE_BATCH];
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int i = base + B * k + threadIdx.x;
+        ev[k] = u[k] = -1;
+        ei[k] = 0;
+        if (i < total) {
+          const int id = upper_bound(s_scan, B, i) - 1;
+          ev[k] = s_v[id];
+          ei[k] = s_st[id] + (i - s_scan[id]);
+          u[k] = __ldg(g.dg_adj_list + ei[k]);
+        }
       }
-      if (FUSED) stage.push(tp, u);
+      push_edges<FUSED>(as, g, f, conf, ev, u, ei, tp);
+      if (FUSED)
+#pragma unroll
+        for (int k = 0; k < EDGE_BATCH; ++k) stage.push(tp[k], u[k]);
     }
     __syncthreads();
   }
@@ -690,8 +750,10 @@ template <bool FUSED, int T, typename G, typename F, typename Src>
 __device__ __forceinline__ void push_strict_body(active_set_t &as, const G &g, F &f, const config_t &conf,
                                                  const Src &src, int64_t n, const int64_t *eoff, const int *tile_lo,
                                                  warp_stage_t &stage) {
+  // per vertex of the tile: itself, its first slot from the tile's first (0 for
+  // one that began earlier) and the column of the tile's first slot, were it its
   __shared__ int s_v[T + 2];
-  __shared__ int64_t s_sc[T + 2];
+  __shared__ int s_sc[T + 2];
   __shared__ int64_t s_st[T + 2];
   const int64_t total = eoff[n];
   const int64_t ntiles = (total + T - 1) / T;
@@ -700,34 +762,40 @@ __device__ __forceinline__ void push_strict_body(active_set_t &as, const G &g, F
     const int64_t lo = tile_lo[t];
     const int64_t hi = (t + 1 < ntiles) ? tile_lo[t + 1] : n - 1;
     const int cnt = (int)(hi - lo + 1);
+    const int64_t t0 = t * T;
     for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
       const int v = src(lo + j);
+      const int64_t at = eoff[lo + j] - t0;
       s_v[j] = v;
-      s_sc[j] = eoff[lo + j];
-      s_st[j] = v >= 0 ? __ldg(g.dg_row_off + v) : 0;
+      s_sc[j] = at < 0 ? 0 : (int)at;
+      s_st[j] = (v >= 0 ? __ldg(g.dg_row_off + v) : 0) - at;
     }
-    if (threadIdx.x == 0) s_sc[cnt] = eoff[hi + 1];
+    // a vertex that goes on past the tile has no end slot in it
+    if (threadIdx.x == 0) s_sc[cnt] = (int)MIN(eoff[hi + 1] - t0, (int64_t)T + 1);
     __syncthreads();
-    const int64_t t0 = t * T;
-    const int64_t t1 = MIN(total, t0 + T);
+    const int ts = (int)MIN(total - t0, (int64_t)T);
+    for (int k0 = 0; k0 < T / EXPAND_THREADS; k0 += EDGE_BATCH) {
+      int ev[EDGE_BATCH], u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool tp[EDGE_BATCH];
 #pragma unroll
-    for (int k = 0; k < T / EXPAND_THREADS; ++k) {
-      const int64_t s = t0 + k * EXPAND_THREADS + threadIdx.x;
-      bool tp = false;
-      int u = -1;
-      if (s < t1) {
-        const int j = upper_bound(s_sc, cnt, s) - 1;
-        const int64_t local = s - s_sc[j];
-        if (local < s_sc[j + 1] - s_sc[j] - 1) {
-          const int64_t ei = s_st[j] + local;
-          u = __ldg(g.dg_adj_list + ei);
-          if (FUSED)
-            tp = push_edge_fused(as, g, f, conf, s_v[j], u, ei);
-          else
-            push_edge_std(as, g, f, conf, s_v[j], u, ei);
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int s = (k0 + k) * EXPAND_THREADS + threadIdx.x;
+        ev[k] = u[k] = -1;
+        ei[k] = 0;
+        if (s < ts) {
+          const int j = upper_bound(s_sc, cnt, s) - 1;
+          if (s < s_sc[j + 1] - 1) {  // not the vertex's end slot
+            ev[k] = s_v[j];
+            ei[k] = s_st[j] + s;
+            u[k] = __ldg(g.dg_adj_list + ei[k]);
+          }
         }
       }
-      if (FUSED) stage.push(tp, u);
+      push_edges<FUSED>(as, g, f, conf, ev, u, ei, tp);
+      if (FUSED)
+#pragma unroll
+        for (int k = 0; k < EDGE_BATCH; ++k) stage.push(tp[k], u[k]);
     }
     __syncthreads();
   }
@@ -1362,20 +1430,26 @@ __device__ __forceinline__ void push_twc_body(active_set_t &as, const G &g, F &f
     s_v[threadIdx.x] = v;
     s_st[threadIdx.x] = st;
     __syncthreads();
-    for (int base = 0; base < total; base += B) {
-      const int i = base + threadIdx.x;
-      bool tp = false;
-      int u = -1;
-      if (i < total) {
-        const int id = upper_bound(s_scan, B, i) - 1;
-        const int64_t ei = s_st[id] + (i - s_scan[id]);
-        u = __ldg(g.dg_adj_list + ei);
-        if (FUSED)
-          tp = push_edge_fused(as, g, f, conf, s_v[id], u, ei);
-        else
-          push_edge_std(as, g, f, conf, s_v[id], u, ei);
+    for (int base = 0; base < total; base += B * EDGE_BATCH) {
+      int ev[EDGE_BATCH], u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool tp[EDGE_BATCH];
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int i = base + B * k + threadIdx.x;
+        ev[k] = u[k] = -1;
+        ei[k] = 0;
+        if (i < total) {
+          const int id = upper_bound(s_scan, B, i) - 1;
+          ev[k] = s_v[id];
+          ei[k] = s_st[id] + (i - s_scan[id]);
+          u[k] = __ldg(g.dg_adj_list + ei[k]);
+        }
       }
-      if (FUSED) stage.push(tp, u);
+      push_edges<FUSED>(as, g, f, conf, ev, u, ei, tp);
+      if (FUSED)
+#pragma unroll
+        for (int k = 0; k < EDGE_BATCH; ++k) stage.push(tp[k], u[k]);
     }
     __syncthreads();
   }
