@@ -305,10 +305,11 @@ struct inspector_t {
     // the push max counter sums per-thread maxima, so it bounds the largest
     // active degree from above; the first level has only its workload
     raw_max_push = c.max_push > 0 ? c.max_push : c.push;
+    raw_max_pull = c.max_pull > 0 ? c.max_pull : c.pull;  // likewise, summed over blocks
   }
 
   // raw counters of the last inspection (before cross() folding)
-  int64_t raw_frontier = 0, raw_inactive = 0, raw_push = 0, raw_pull = 0, raw_max_push = 0;
+  int64_t raw_frontier = 0, raw_inactive = 0, raw_push = 0, raw_pull = 0, raw_max_push = 0, raw_max_pull = 0;
 };
 
 // ===========================================================================
@@ -628,6 +629,8 @@ struct executor_t {
                  as.fmt == Queue)
                     ? insp->raw_max_push
                     : -1;
+    if (!conf.conf_fuse_inspect && insp && conf.conf_dir == Pull && conf.conf_target == Inactive)
+      h.max_deg = insp->raw_max_pull;
   }
 
   // deferred filter updates of fused levels (kernel_fusion.cuh:54-109)
@@ -846,8 +849,15 @@ struct executor_t {
       }
     } else {
       switch (conf.conf_lb) {
-        case WM: GSW_GO((k_pull_wm<G, F>), fr < 0 ? -1 : fr / B + 1, as, g, f, conf); break;
-        case CM: GSW_GO((k_pull_cm<G, F>), fr < 0 ? -1 : fr / B + 1, as, g, f, conf); break;
+        case WM:
+        case CM: {
+          const hub_list_t hl = hub_list_for(as, g, conf.conf_lb == WM ? WM_HUB_MIN : CM_HUB_MIN);
+          if (!ok()) return;
+          if (conf.conf_lb == WM) GSW_GO((k_pull_wm<G, F>), fr < 0 ? -1 : fr / B + 1, as, g, f, conf, hl);
+          else GSW_GO((k_pull_cm<G, F>), fr < 0 ? -1 : fr / B + 1, as, g, f, conf, hl);
+          if (hl.piece) GSW_GO((k_pull_hubs<G, F>), -1, as, g, f, conf, hl);
+          break;
+        }
         case TWC: GSW_GO((k_pull_twc<G, F>), fr < 0 ? -1 : fr / B + 1, as, g, f, conf); break;
         case STRICT: {
           // from-all pulls stage a per-vertex sum too: their tiles stop at

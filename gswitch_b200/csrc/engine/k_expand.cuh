@@ -449,11 +449,51 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_push_wm(active_set_t as, G g
   if (FUSED) stage.flush();
 }
 
+// The messages of EDGE_BATCH in-edges of a thread (u < 0: none), step by step
+// over all of them as in push_edges: which senders are active, then what they send
 template <typename G, typename F>
-__global__ void __launch_bounds__(EXPAND_THREADS) k_pull_wm(active_set_t as, G g, F f, config_t conf) {
+__device__ __forceinline__ void pull_edges(const active_set_t &as, const G &g, F &f, const config_t &conf,
+                                           const int (&u)[EDGE_BATCH], const int64_t (&ei)[EDGE_BATCH],
+                                           bool (&have)[EDGE_BATCH], typename F::wa_t (&x)[EDGE_BATCH]) {
+#pragma unroll
+  for (int k = 0; k < EDGE_BATCH; ++k) have[k] = u[k] >= 0 && (conf.conf_fromall || as.bitmap.is_active(u[k]));
+#pragma unroll
+  for (int k = 0; k < EDGE_BATCH; ++k)
+    x[k] = have[k] ? f.emit(u[k], g.fetch_edata_r(ei[k]), g) : typename F::wa_t();
+}
+
+// Folds the messages of each run of lanes with the same id into its first lane;
+// true there if the run has a message.  Every lane of the warp calls it.
+template <typename WA, typename G, typename F>
+__device__ __forceinline__ bool fold_runs(F &f, const G &g, int id, bool have, WA &io) {
+  // by value: clearing the array of messages with memset and folding in place,
+  // nvcc 12.9 lost updates of a mixed int/float message (BCBackward)
+  WA x = io;
+  const int lane = lane_id();
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int oid = __shfl_down_sync(FULL, id, d);
+    const bool oh = __shfl_down_sync(FULL, have, d);
+    const WA ox = shfl_down_any(x, d);
+    if (lane + d < 32 && oid == id && oh) {
+      if (have)
+        f.comp(&x, ox, g);
+      else
+        x = ox;
+      have = true;
+    }
+  }
+  io = x;
+  const int pid = __shfl_up_sync(FULL, id, 1);
+  return have && (lane == 0 || pid != id);
+}
+
+template <typename G, typename F>
+__global__ void __launch_bounds__(EXPAND_THREADS) k_pull_wm(active_set_t as, G g, F f, config_t conf,
+                                                            hub_list_t hubs) {
   using WA = typename F::wa_t;
   constexpr int W = EXPAND_THREADS / 32;
-  __shared__ int s_scan[W][33];
+  __shared__ int s_scan[W][32];
   __shared__ int s_v[W][32];
   __shared__ int64_t s_st[W][32];
   const int64_t n = as.get_size();
@@ -467,48 +507,38 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_wm(active_set_t as, G g
     int64_t st;
     int deg;
     vertex_range(g, true, v, st, deg);
+    if (defer_hub(as, conf, hubs, v, st, deg, WM_HUB_MIN)) deg = 0;
     const int incl = warp_inclusive_sum(deg);
     const int total = __shfl_sync(FULL, incl, 31);
     if (lane == 0) account(as, conf, (unsigned long long)total);
     s_scan[w][lane] = incl - deg;
-    if (lane == 31) s_scan[w][32] = total;
     s_v[w][lane] = v;
     s_st[w][lane] = st;
     __syncwarp();
-    for (int base = 0; base < total; base += 32) {
-      const int i = base + lane;
-      int id = 31;
-      bool vote = false;
-      WA val;
-      memset(&val, 0, sizeof(WA));
-      if (i < total) {
-        id = upper_bound(s_scan[w], 32, i) - 1;
-        const int64_t ei = s_st[w][id] + (i - s_scan[w][id]);
-        const int u = __ldg(g.dgr_adj_list + ei);
-        if (conf.conf_fromall || as.bitmap.is_active(u)) {
-          vote = true;
-          val = f.emit(u, g.fetch_edata_r(ei), g);
-        }
-      } else {
-        id = 32 + lane;  // past-the-end lanes form their own segments
-      }
-      // segmented reduction toward the first lane of each owner's run
+    for (int base = 0; base < total; base += 32 * EDGE_BATCH) {
+      int id[EDGE_BATCH], u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool have[EDGE_BATCH];
+      WA x[EDGE_BATCH];
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int oid = __shfl_down_sync(FULL, id, d);
-        const bool ovote = __shfl_down_sync(FULL, vote, d);
-        const WA oval = shfl_down_any(val, d);
-        if (lane + d < 32 && oid == id && ovote) {
-          if (vote)
-            f.comp(&val, oval, g);
-          else
-            val = oval;
-          vote = true;
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int i = base + 32 * k + lane;
+        id[k] = 32 + lane;  // past-the-end lanes form their own runs
+        u[k] = -1;
+        ei[k] = 0;
+        if (i < total) {
+          id[k] = upper_bound(s_scan[w], 32, i) - 1;
+          ei[k] = s_st[w][id[k]] + (i - s_scan[w][id[k]]);
+          u[k] = __ldg(g.dgr_adj_list + ei[k]);
         }
       }
-      const int pid = __shfl_up_sync(FULL, id, 1);
-      const bool head = (lane == 0) || (pid != id);
-      if (i < total && head && vote) f.comp(f.wa_of(s_v[w][id]), val, g);
+      pull_edges(as, g, f, conf, u, ei, have, x);
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        if (!__any_sync(FULL, have[k])) continue;
+        if (fold_runs(f, g, id[k], have[k], x[k])) f.comp(f.wa_of(s_v[w][id[k]]), x[k], g);
+        __syncwarp();  // a vertex's next run may sit in another lane
+      }
     }
     __syncwarp();
   }
@@ -576,8 +606,13 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_push_cm(active_set_t as, G g
   if (FUSED) stage.flush();
 }
 
+// The messages of a warp's 32 edges meet in registers first: with an atomic an
+// edge, a hub's all went to one address (4.2 ms for one backward level of
+// betweenness on RMAT 2^20).
 template <typename G, typename F>
-__global__ void __launch_bounds__(EXPAND_THREADS) k_pull_cm(active_set_t as, G g, F f, config_t conf) {
+__global__ void __launch_bounds__(EXPAND_THREADS) k_pull_cm(active_set_t as, G g, F f, config_t conf,
+                                                            hub_list_t hubs) {
+  using WA = typename F::wa_t;
   constexpr int B = EXPAND_THREADS;
   __shared__ int s_scan[B];
   __shared__ int s_v[B];
@@ -592,6 +627,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_cm(active_set_t as, G g
     int64_t st;
     int deg;
     vertex_range(g, true, v, st, deg);
+    if (defer_hub(as, conf, hubs, v, st, deg, CM_HUB_MIN)) deg = 0;
     int total;
     const int ex = block_exclusive_scan(deg, s_tmp, &total);
     if (threadIdx.x == 0) account(as, conf, (unsigned long long)total);
@@ -599,17 +635,91 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_cm(active_set_t as, G g
     s_v[threadIdx.x] = v;
     s_st[threadIdx.x] = st;
     __syncthreads();
-    for (int base = 0; base < total; base += B) {
-      const int i = base + threadIdx.x;
-      if (i < total) {
-        const int id = upper_bound(s_scan, B, i) - 1;
-        const int64_t ei = s_st[id] + (i - s_scan[id]);
-        const int u = __ldg(g.dgr_adj_list + ei);
-        if (conf.conf_fromall || as.bitmap.is_active(u)) {
-          auto vd = f.emit(u, g.fetch_edata_r(ei), g);
-          f.compAtomic(f.wa_of(s_v[id]), vd, g);
+    for (int base = 0; base < total; base += B * EDGE_BATCH) {
+      int id[EDGE_BATCH], u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool have[EDGE_BATCH];
+      WA x[EDGE_BATCH];
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int i = base + B * k + threadIdx.x;
+        id[k] = B + lane_id();
+        u[k] = -1;
+        ei[k] = 0;
+        if (i < total) {
+          id[k] = upper_bound(s_scan, B, i) - 1;
+          ei[k] = s_st[id[k]] + (i - s_scan[id[k]]);
+          u[k] = __ldg(g.dgr_adj_list + ei[k]);
         }
       }
+      pull_edges(as, g, f, conf, u, ei, have, x);
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        if (!__any_sync(FULL, have[k])) continue;
+        if (fold_runs(f, g, id[k], have[k], x[k])) f.compAtomic(f.wa_of(s_v[id[k]]), x[k], g);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// the hub pieces a warp- or CTA-mapped pull listed: a CTA folds a piece into
+// one message (with a hub on the one warp that found it, the widest backward
+// level of betweenness on RMAT 2^20 took 482 us; 83 us with its pieces spread)
+template <typename G, typename F>
+__global__ void __launch_bounds__(EXPAND_THREADS) k_pull_hubs(active_set_t as, G g, F f, config_t conf,
+                                                              hub_list_t hubs) {
+  using WA = typename F::wa_t;
+  constexpr int B = EXPAND_THREADS, NW = B / 32;
+  __shared__ WA s_part[NW];
+  __shared__ int s_have[NW];
+  __shared__ int s_np;
+  if (threadIdx.x == 0) {
+    s_np = (int)MIN((int64_t)*(volatile int *)hubs.count, hubs.cap);
+    __threadfence();
+    if (atomicAdd(hubs.done, 1u) == gridDim.x - 1) {  // every CTA has read the count
+      *hubs.count = 0;
+      *hubs.done = 0;
+    }
+  }
+  __syncthreads();
+  const int np = s_np, lane = lane_id();
+  for (int p = blockIdx.x; p < np; p += gridDim.x) {
+    const hub_piece_t pc = hubs.piece[p];
+    WA acc = WA();
+    bool any = false;
+    for (int base = 0; base < pc.len; base += B * EDGE_BATCH) {
+      int u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool have[EDGE_BATCH];
+      WA x[EDGE_BATCH];
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int i = base + B * k + threadIdx.x;
+        ei[k] = pc.st + i;
+        u[k] = i < pc.len ? __ldg(g.dgr_adj_list + ei[k]) : -1;
+      }
+      pull_edges(as, g, f, conf, u, ei, have, x);
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        if (!have[k]) continue;
+        if (any)
+          f.comp(&acc, x[k], g);
+        else
+          acc = x[k];
+        any = true;
+      }
+    }
+    const bool has = fold_runs(f, g, 0, any, acc);
+    if (lane == 0) {
+      s_part[warp_id()] = acc;
+      s_have[warp_id()] = has;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      WA y = s_part[lane < NW ? lane : 0];
+      const bool yh = lane < NW && s_have[lane];
+      if (fold_runs(f, g, 0, yh, y)) f.compAtomic(f.wa_of(pc.v), y, g);
     }
     __syncthreads();
   }
@@ -827,9 +937,9 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_strict(active_set_t as,
                                                                 const int *tile_lo) {
   using WA = typename F::wa_t;
   constexpr int B = EXPAND_THREADS;
-  constexpr int PER = T / B;
+  // as in push_strict_body, on in-edges
   __shared__ int s_v[T + 2];
-  __shared__ int64_t s_sc[T + 2];
+  __shared__ int s_sc[T + 2];
   __shared__ int64_t s_st[T + 2];
   const int64_t n = as.get_size();
   GSW_HALT_IF_EMPTY(n);
@@ -837,65 +947,55 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_strict(active_set_t as,
   const int64_t *eoff = as.workset.dg_eoff;
   const int64_t total = eoff[n];
   const int64_t ntiles = (total + T - 1) / T;
-  const int lane = lane_id();
   if (blockIdx.x == 0 && threadIdx.x == 0) account(as, conf, (unsigned long long)(total - n));
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int64_t lo = tile_lo[t];
     const int64_t hi = (t + 1 < ntiles) ? tile_lo[t + 1] : n - 1;
     const int cnt = (int)(hi - lo + 1);
+    const int64_t t0 = t * T;
+    const bool cut = eoff[lo] < t0;  // the tile's first vertex began earlier
     for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
       const int v = as.fetch(lo + j, want);
+      const int64_t at = eoff[lo + j] - t0;
       s_v[j] = v;
-      s_sc[j] = eoff[lo + j];
-      s_st[j] = v >= 0 ? __ldg(g.dgr_row_off + v) : 0;
+      s_sc[j] = at < 0 ? 0 : (int)at;
+      s_st[j] = (v >= 0 ? __ldg(g.dgr_row_off + v) : 0) - at;
     }
-    if (threadIdx.x == 0) s_sc[cnt] = eoff[hi + 1];
+    // T + 2: its edges go on past the tile; T + 1: only its end slot lies there
+    if (threadIdx.x == 0) s_sc[cnt] = (int)MIN(eoff[hi + 1] - t0, (int64_t)T + 2);
     __syncthreads();
-    const int64_t t1 = MIN(total, t * T + T);
-    for (int k = 0; k < PER; ++k) {
-      const int64_t wbase = t * T + (int64_t)k * B + (threadIdx.x & ~31);
-      if (wbase >= t1) break;  // warp-uniform
-      const int64_t s = wbase + lane;
-      int j = -1;
-      bool have = false;
-      WA x = f.data.zero;
-      if (s < t1) {
-        j = upper_bound(s_sc, cnt, s) - 1;
-        const int64_t local = s - s_sc[j];
-        if (local < s_sc[j + 1] - s_sc[j] - 1) {
-          const int64_t ei = s_st[j] + local;
-          const int u = __ldg(g.dgr_adj_list + ei);
-          if (conf.conf_fromall || as.bitmap.is_active(u)) {
-            x = f.emit(u, g.fetch_edata_r(ei), g);
-            have = true;
-          }
-        }
-      }
-      // segmented inclusive scan over runs of equal j (j is non-decreasing
-      // across the lanes)
+    const int ts = (int)MIN(total - t0, (int64_t)T);
+    for (int k0 = 0; k0 < T / B; k0 += EDGE_BATCH) {
+      int id[EDGE_BATCH], u[EDGE_BATCH];
+      int64_t ei[EDGE_BATCH];
+      bool have[EDGE_BATCH];
+      WA x[EDGE_BATCH];
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const WA ox = shfl_up_any(x, d);
-        const int oj = __shfl_up_sync(FULL, j, d);
-        const bool oh = __shfl_up_sync(FULL, have ? 1 : 0, d) != 0;
-        if (lane >= d && oj == j && oh) {
-          if (have) {
-            f.comp(&x, ox, g);
-          } else {
-            x = ox;
-            have = true;
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        const int s = (k0 + k) * B + threadIdx.x;
+        id[k] = cnt + lane_id();
+        u[k] = -1;
+        ei[k] = 0;
+        if (s < ts) {
+          id[k] = upper_bound(s_sc, cnt, s) - 1;
+          if (s < s_sc[id[k] + 1] - 1) {  // not the vertex's end slot
+            ei[k] = s_st[id[k]] + s;
+            u[k] = __ldg(g.dgr_adj_list + ei[k]);
           }
         }
       }
-      const int nj = __shfl_down_sync(FULL, j, 1);
-      const bool tail = lane == 31 || nj != j;
-      if (tail && have && j >= 0) {
-        const int64_t first = s_sc[j];
-        const int64_t last = s_sc[j + 1] - 2;  // the vertex's last edge slot
-        if (first >= wbase && last <= wbase + 31)
-          f.comp(f.wa_of(s_v[j]), x, g);
+      pull_edges(as, g, f, conf, u, ei, have, x);
+#pragma unroll
+      for (int k = 0; k < EDGE_BATCH; ++k) {
+        if (!__any_sync(FULL, have[k])) continue;
+        if (!fold_runs(f, g, id[k], have[k], x[k])) continue;
+        // one write when all of the vertex's edges sit in this warp's 32 slots
+        const int w0 = (k0 + k) * B + (threadIdx.x & ~31);
+        const bool whole = s_sc[id[k]] >= w0 && s_sc[id[k] + 1] - 2 <= w0 + 31 && !(cut && id[k] == 0);
+        if (whole)
+          f.comp(f.wa_of(s_v[id[k]]), x[k], g);
         else
-          f.compAtomic(f.wa_of(s_v[j]), x, g);
+          f.compAtomic(f.wa_of(s_v[id[k]]), x[k], g);
       }
     }
     __syncthreads();
