@@ -22,6 +22,7 @@
 #include "engine/mlp.cuh"
 #include "graphgen.cuh"
 #include "bc_batch.cuh"
+#include "bfs_small.cuh"
 #include "cc_forest.cuh"
 #include "gc_dag.cuh"
 #include "mbfs.cuh"
@@ -93,6 +94,12 @@ struct gsw_ctx {
   mlp_model mlp{};                // learned selector (valid = 0: none loaded)
   mlp_model mlp_fusion{};         // learned fusion decision of Mono-pattern runs
   mlp_model *dmlp = nullptr;      // its device copy (captured loops)
+  // what a run leaves behind, in pinned memory: read with the run's one wait
+  struct run_report {
+    sb_state_t small;            // the state of a small BFS
+    unsigned err;                // the active set's error word
+    unsigned long long reached;  // degree sum of the reached vertices
+  } *report = nullptr;
   std::string record_path;        // per-level feature records (empty: off)
 
   // Device blocks of destroyed graphs, kept for the next graph of a fitting
@@ -782,8 +789,13 @@ struct timer {
     cudaEventRecord(ctx->e0, stream());
   }
   double stop() {
-    cudaEventRecord(ctx->e1, stream());
+    mark();
     cudaEventSynchronize(ctx->e1);
+    return elapsed();
+  }
+  // the end without waiting for it; elapsed() once the stream has been waited for
+  void mark() { cudaEventRecord(ctx->e1, stream()); }
+  double elapsed() {
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->e0, ctx->e1);
     return ms;
@@ -807,8 +819,11 @@ void add_persistent_levels(gsw_run_stats *st, executor_t &ex, int64_t lv0, int64
   if (st) st->levels += (int)((ex.persistent_levels - lv0) - (ex.persistent_launches - ln0));
 }
 
-unsigned end_checks(active_set_t *as, gsw_run_stats *st) {
-  const unsigned e = as->read_error();
+bool ensure_report(gsw_ctx *ctx) {
+  return ctx->report || GSW_CUDA(cudaMallocHost((void **)&ctx->report, sizeof(*ctx->report))) == 0;
+}
+
+void end_checks(unsigned e, active_set_t *as, gsw_run_stats *st) {
   if (st) {
     st->device_error = e;
     st->launches = launch_count();
@@ -818,9 +833,31 @@ unsigned end_checks(active_set_t *as, gsw_run_stats *st) {
   if (e & DEV_ERR_BARRIER_TIMEOUT) set_error(GSW_ERR_TIMEOUT, "%s", "grid barrier timed out");
   if (e & DEV_ERR_STAGE_TIMEOUT) set_error(GSW_ERR_TIMEOUT, "%s", "shared-memory staging copy did not complete");
   if (e & DEV_ERR_BAD_VERTEX) set_error(GSW_ERR_CUDA, "%s", "pointer chain longer than n");
-  GSW_CUDA(cudaMemsetAsync(&as->dg_cnt->err, 0, sizeof(unsigned), stream()));
-  return e;
+  if (e) GSW_CUDA(cudaMemsetAsync(&as->dg_cnt->err, 0, sizeof(unsigned), stream()));
 }
+void end_checks(active_set_t *as, gsw_run_stats *st) { end_checks(as->read_error(), as, st); }
+
+// The end of a run over vertex values: the device time, the error word and the
+// traversed edges come back with one wait (each waited on its own before).
+void end_run(gsw_ctx *ctx, gsw_graph *gr, active_set_t *as, timer &tm, const int *vals, int unreached,
+             gsw_run_stats *st) {  // after tm.mark()
+  if (!ensure_report(ctx)) return;
+  GSW_CUDA(cudaMemcpyAsync(&ctx->report->err, &as->dg_cnt->err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream()));
+  if (st) {
+    unsigned long long *d = (unsigned long long *)ctx->buf("redges", 8);
+    if (!d) return;
+    GSW_CUDA(cudaMemsetAsync(d, 0, 8, stream()));
+    k_reached_edges<<<grid_for(gr->n), 256, 0, stream()>>>(vals, 1, unreached, gr->odeg, gr->n, d);
+    GSW_CUDA(cudaMemcpyAsync(&ctx->report->reached, d, 8, cudaMemcpyDeviceToHost, stream()));
+  }
+  GSW_CUDA(cudaStreamSynchronize(stream()));
+  end_checks(ctx->report->err, as, st);
+  if (st) {
+    st->ms = tm.elapsed();
+    st->edges = (int64_t)(ctx->report->reached / 2);
+  }
+}
+
 
 // level cap of every loop: far above any legitimate run, it turns a loop
 // that cannot converge into an error instead of a hang
@@ -1199,6 +1236,7 @@ gsw_status gsw_destroy(gsw_ctx *ctx) {
   for (auto &kv : ctx->dl) kv.second.destroy();
   cudaFree(ctx->dtrees);
   cudaFree(ctx->dmlp);
+  if (ctx->report) cudaFreeHost(ctx->report);
   ctx->executor.destroy();
   ctx->stats.destroy();
   if (ctx->e0) cudaEventDestroy(ctx->e0);
@@ -1554,6 +1592,61 @@ gsw_status gsw_ctx_stream(gsw_ctx *ctx, void **s) {
 // ---------------------------------------------------------------------------
 // BFS: application/bfs.cu:78-102 (loop) and :104-130 (set-up)
 // ---------------------------------------------------------------------------
+// Nothing about the level loop is asked for: no forced choice, no per-level
+// record, no per-launch form; nor, unless the caller says so, the captured one.
+static bool unforced(const gsw_run_opts *o, bool captured_too = false) {
+  return !record_sink() && !g_label &&
+         (!o || (o->direction < 0 && o->asfmt < 0 && o->lb < 0 && o->fusion < 0 && !o->verbose && !o->timing &&
+                 o->expand_grid == 0 && !o->account && o->persistent != 0 && !o->barrier_test &&
+                 (captured_too || !o->captured)));
+}
+
+// a small graph's BFS in one launch (bfs_small.cuh): the loop's levels and
+// traversed edges
+static gsw_status bfs_small_run(gsw_ctx *ctx, gsw_graph *gr, const int32_t *roots, int nroots, int32_t *levels,
+                                gsw_run_stats *st, entry_guard &eg) {
+  const size_t room = sizeof(sb_piece_t) * (size_t)(gr->n + gr->m / SB_PIECE + 2);
+  int *lvl = (int *)ctx->buf("wa", sizeof(int) * (gr->n + 1));
+  sb_piece_t *q0 = (sb_piece_t *)ctx->buf("sb_q0", room), *q1 = (sb_piece_t *)ctx->buf("sb_q1", room);
+  sb_state_t *S = (sb_state_t *)ctx->buf("sb_state", sizeof(sb_state_t));
+  if (!lvl || !q0 || !q1 || !S) return eg.finish();
+  int *droots = nullptr, root = roots[0];
+  if (nroots > 1) {
+    droots = (int *)ctx->buf("bfs_roots", sizeof(int) * nroots);
+    if (!droots) return eg.finish();
+    GSW_CUDA(cudaMemcpyAsync(droots, roots, sizeof(int) * nroots, cudaMemcpyHostToDevice, stream()));
+  }
+  auto g = gr->view<Empty>();
+  unsigned long long budget = 2000000000ull;  // per barrier wait
+  // no more CTAs than the widest level can use, and a cheaper barrier for it
+  const int grid = clamp_grid(gr->m / (4 * SB_THREADS) + 1, resident_grid(k_bfs_small, SB_THREADS));
+  if (!ensure_report(ctx)) return eg.finish();
+  GSW_CUDA(cudaMemsetAsync(S, 0, sizeof(sb_state_t), stream()));
+  timer tm(ctx);
+  void *args[] = {(void *)&g,  (void *)&root, (void *)&droots, (void *)&nroots, (void *)&lvl,
+                  (void *)&q0, (void *)&q1,   (void *)&S,      (void *)&budget};
+  if (!GSW_CUDA(cudaLaunchCooperativeKernel((const void *)k_bfs_small, grid, SB_THREADS, args, 0, stream())))
+    GSW_LAUNCHED();
+  tm.mark();
+  GSW_CUDA(cudaMemcpyAsync(&ctx->report->small, S, sizeof(sb_state_t), cudaMemcpyDeviceToHost, stream()));
+  if (levels && ok()) GSW_CUDA(cudaMemcpyAsync(levels, lvl, sizeof(int) * gr->n, cudaMemcpyDeviceToHost, stream()));
+  GSW_CUDA(cudaStreamSynchronize(stream()));
+  if (!ok()) return eg.finish();
+  if (ctx->report->small.status == 2) set_error(GSW_ERR_TIMEOUT, "%s", "grid barrier timed out");
+  if (st) {
+    st->ms = tm.elapsed();
+    st->levels = ctx->report->small.levels;
+    st->edges = (int64_t)(ctx->report->small.reached / 2);
+    st->launches = launch_count();
+    st->level_cfg[0] = ((int)WM << 2) | (1 << 5) | (1 << 6);  // one persistent launch: push, queue, warps
+    st->level_frontier[0] = -1;
+    st->level_ms[0] = st->level_inspect_ms[0] = 0;
+    st->level_edges[0] = 0;
+    st->ntrace = 1;
+  }
+  return eg.finish();
+}
+
 // BFS from one root, or from several at once (levels = distance to the
 // nearest root; over a disjoint union of graphs with one root per part this
 // is one BFS per part, all in the same level loop)
@@ -1561,6 +1654,9 @@ gsw_status bfs_run(gsw_ctx *ctx, gsw_graph *gr, const int32_t *roots, int nroots
                    int32_t *levels, gsw_run_stats *st, entry_guard &eg) {
   const int32_t root = roots[0];
   begin_stats(st);
+  // the captured form too: like the graph, the launch needs no host until the answer
+  if (unforced(o, true) && gr->n <= SB_MAX_VERTICES && gr->m <= SB_MAX_ARCS)
+    return bfs_small_run(ctx, gr, roots, nroots, levels, st, eg);
   auto g = gr->view<Empty>();
   app::BFS f;
   f.data.size = gr->n;
@@ -1568,8 +1664,8 @@ gsw_status bfs_run(gsw_ctx *ctx, gsw_graph *gr, const int32_t *roots, int nroots
   if (!f.data.dg_wa) return eg.finish();
   int64_t root_degree_sum = 0;
   if (nroots == 1) {
+    root_degree_sum = root_deg(gr, root);  // before the fill: the host waits for this copy only
     fill_root<int>(f.data.dg_wa, -1, 0, root, gr->n);
-    root_degree_sum = root_deg(gr, root);
   } else {
     int *droots = (int *)ctx->buf("bfs_roots", sizeof(int) * nroots);
     if (!droots) return eg.finish();
@@ -1631,15 +1727,11 @@ gsw_status bfs_run(gsw_ctx *ctx, gsw_graph *gr, const int32_t *roots, int nroots
     tr.done(stats, fets);
     if (finish(as, g, f, conf)) break;
   }
-  const double ms = tm.stop();
+  tm.mark();
   if (captured) dl_collect(R, st);
+  end_run(ctx, gr, &as, tm, f.data.dg_wa, -1, st);
   tr.resolve();
-  end_checks(&as, st);
   add_persistent_levels(st, executor, plv0, pln0);
-  if (st) {
-    st->ms = ms;
-    st->edges = reached_edges(ctx, gr, f.data.dg_wa, 1, -1);
-  }
   if (levels && ok())
     GSW_CUDA(cudaMemcpyAsync(levels, f.data.dg_wa, sizeof(int) * gr->n, cudaMemcpyDeviceToHost, stream()));
   GSW_CUDA(cudaStreamSynchronize(stream()));
@@ -1873,6 +1965,7 @@ gsw_status gsw_sssp(gsw_ctx *ctx, gsw_graph *gr, int32_t root, const gsw_run_opt
   f.data.dg_wa = (int *)ctx->buf("wa", sizeof(int) * (gr->n + 1));
   f.data.dg_ra = (int *)ctx->buf("ra", sizeof(int) * (gr->n + 1));
   if (!f.data.dg_wa || !f.data.dg_ra) return eg.finish();
+  const int64_t rdeg = root_deg(gr, root);  // before the fills: the host waits for this copy only
   fill_root<int>(f.data.dg_wa, INT_MAX, 0, root, gr->n);
   fill_root<int>(f.data.dg_ra, INT_MAX, 0, root, gr->n);
   feature_t fets;
@@ -1893,7 +1986,7 @@ gsw_status gsw_sssp(gsw_ctx *ctx, gsw_graph *gr, int32_t root, const gsw_run_opt
   apply_opts(o, conf);
   set_graph_features(fets, gr);
   fets.use_root = root;
-  init_conf_impl(stats, fets, conf, g, f, gr->mean_weight, gr->attr[0], false, root_deg(gr, root));
+  init_conf_impl(stats, fets, conf, g, f, gr->mean_weight, gr->attr[0], false, rdeg);
   mlp_fusion_override(ctx, o, fets, conf);
   active_set_t *asp = ctx->aset(gr->n, conf.conf_qmode);
   if (!asp) return eg.finish();
@@ -1919,15 +2012,11 @@ gsw_status gsw_sssp(gsw_ctx *ctx, gsw_graph *gr, int32_t root, const gsw_run_opt
     tr.done(stats, fets);
     if (finish(as, g, f, conf)) break;
   }
-  const double ms = tm.stop();
+  tm.mark();
   if (captured) dl_collect(R, st);
+  end_run(ctx, gr, &as, tm, f.data.dg_wa, INT_MAX, st);
   tr.resolve();
-  end_checks(&as, st);
   add_persistent_levels(st, executor, plv0, pln0);
-  if (st) {
-    st->ms = ms;
-    st->edges = reached_edges(ctx, gr, f.data.dg_wa, 1, INT_MAX);
-  }
   if (dist && ok()) GSW_CUDA(cudaMemcpyAsync(dist, f.data.dg_wa, sizeof(int) * gr->n, cudaMemcpyDeviceToHost, stream()));
   GSW_CUDA(cudaStreamSynchronize(stream()));
   return eg.finish();
@@ -2111,14 +2200,6 @@ static bool cc_captured_run(gsw_ctx *ctx, device_graph_t<COO, Empty> g, app::CC 
     }
   }
   return ok();
-}
-
-// Nothing about the level loop is asked for: no forced choice, no per-level
-// record, no captured or per-launch form.
-static bool unforced(const gsw_run_opts *o) {
-  return !record_sink() && !g_label &&
-         (!o || (o->direction < 0 && o->asfmt < 0 && o->lb < 0 && o->fusion < 0 && !o->verbose && !o->timing &&
-                 o->expand_grid == 0 && !o->account && o->persistent != 0 && !o->barrier_test && !o->captured));
 }
 
 // is the graph stored with every arc listed from both ends? (an undirected

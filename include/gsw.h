@@ -151,7 +151,9 @@ typedef struct gsw_run_opts {
                         device-side selection and termination (BFS, SSSP, PR,
                         delta-PR, CC, GC; GSW_ERR_UNSUPPORTED for BC, MBFS and
                         batched BC, whose batched forms run every level in one
-                        cooperative launch); 0: host-driven loop */
+                        cooperative launch; a small graph's BFS with no forced
+                        choice is one such launch in either form); 0:
+                        host-driven loop */
   int hub_path;      /* how a CTA sweeps one hub's adjacency list (the
                         thread/warp/CTA-tiered push's CTA tier): 0 four-byte
                         loads, 1 int4 loads of the 16-byte-aligned body,
