@@ -496,7 +496,6 @@ bool dl_build(dloop_graph &L, executor_t &ex, dloop_t *d, active_set_t as, devic
   hints().edges = -1;
   hints().max_deg = -1;  // a captured body sweeps whatever hubs its level lists
   ex.ensure_tiles(g.nedges + as.size + 1);
-  ex.ensure_all_tiles(as.size, g.nedges);
   dloop_t &im = L.image;
   im = dloop_t();
   im.persist_fused = persist ? 1 : 0;

@@ -943,7 +943,11 @@ bool dl_prepare(dl_run &R, gsw_ctx *ctx, int app, dl_key key, active_set_t &as, 
   if (!trees || !R.d || !R.trace_cfg || !R.trace_frontier || !R.trace_edges || !R.trace_t || !R.trace_sel)
     return false;
   executor_t &ex = ctx->executor;
+  // every table a body may use, before the capture and in the key: a later run
+  // on a larger graph replaces them
   ex.ensure_tiles(g.nedges + as.size + 1);
+  ex.ensure_all_tiles(as.size, g.nedges);
+  ex.ensure_hubs(g.nedges);
   if (!ok()) return false;
   key << app << R.d << g.dg_row_off << g.dg_adj_list << g.dg_odegree << g.dg_edgedata << g.dgr_row_off
       << g.dgr_adj_list << g.dgr_odegree << g.dgr_edgedata << g.nvertexs << g.nedges << g.directed;
@@ -951,7 +955,7 @@ bool dl_prepare(dl_run &R, gsw_ctx *ctx, int app, dl_key key, active_set_t &as, 
       << as.queue.subqueue[0].dg_queue << as.queue.subqueue[1].dg_queue << as.queue.subqueue[0].max_size
       << as.dg_cnt << as.workset.dg_eoff << as.workset.dg_bsum << as.workset.bsum_cap;
   key << conf.conf_pruning << conf.conf_count_edges << conf.conf_sorted_queue << fets.fromall << fets.toall
-      << ex.dg_tile << ex.tile_cap << ex.twod.edge << opts().force_grid << ctx->stats.dg_runtime_info;
+      << ex.dg_tile << ex.tile_cap << ex.dg_all_tile << ex.all_tile_cap << ex.dg_hubs << ex.hub_cap << ex.twod.edge << opts().force_grid << ctx->stats.dg_runtime_info;
   key << conf.conf_window << conf.conf_fusion << f.data.dg_ra << conf.conf_persistent;
   for (int q : ex.tune.quarters[0][0][0]) key << q;  // first row: cheap change detector
   {
@@ -1635,7 +1639,7 @@ static gsw_status bfs_small_run(gsw_ctx *ctx, gsw_graph *gr, const int32_t *root
   if (ctx->report->small.status == 2) set_error(GSW_ERR_TIMEOUT, "%s", "grid barrier timed out");
   if (st) {
     st->ms = tm.elapsed();
-    st->levels = ctx->report->small.levels;
+    st->levels = std::max(1, ctx->report->small.levels);  // the root's level runs even without arcs
     st->edges = (int64_t)(ctx->report->small.reached / 2);
     st->launches = launch_count();
     st->level_cfg[0] = ((int)WM << 2) | (1 << 5) | (1 << 6);  // one persistent launch: push, queue, warps

@@ -62,3 +62,22 @@ def test_tile_edges(ctx, case, directed):
             assert {t[:3] for t in st.trace} == {tuple(cfg.split("-"))}
             assert np.max(np.abs(pr - ref) / ref) <= bound[cfg[:4]], (name, cfg, captured)
     g.close()
+
+
+def test_captured_graph_outlives_no_table(ctx):
+    """A captured loop, a run on a larger graph that replaces the tables its
+    bodies name, and the captured loop again: it is captured anew."""
+    r = np.random.default_rng(9)
+    small = csr(3000, r.integers(0, 3000, 20000), r.integers(0, 3000, 20000))
+    big = csr(200000, r.integers(0, 200000, 3000000), (r.random(3000000) ** 4 * 200000).astype(np.int64))
+    gs_, gb = (ctx.upload(x[0], x[1], directed=True) for x in (small, big))
+    for cfg in ("Pull-Bitmap-STRICT", "Push-Bitmap-STRICT", "Pull-Bitmap-WM", "Push-Bitmap-CM"):
+        cap = gs.RunOpts.from_config(cfg, captured=True)
+        ref = pagerank(3000, small[0], small[1], small[2], 3)
+        for _ in range(2):
+            pr, _ = gs_.pagerank(iters=3, eps=0.0, opts=cap)
+            # in-degrees below 40: 2.6 * (20 + 40) * 2^-24
+            assert np.max(np.abs(pr - ref) / ref) <= 1e-5, cfg
+            gb.pagerank(iters=2, eps=0.0, opts=cfg, out=False)
+    gs_.close()
+    gb.close()
