@@ -53,13 +53,23 @@ inline int clamp_grid(int64_t want, int cap) {
   return (int)MIN(want, (int64_t)cap);
 }
 
-// the VC inspection on one wave of resident CTAs (no more CTAs than units)
+// the VC inspection, as inspect_plan lays it out
 template <typename G, typename F>
 inline void launch_inspect_vc(const active_set_t &as, const G &g, const F &f, unsigned long long *info,
                               const int *skip_if = nullptr, unsigned long long *sig = nullptr,
                               unsigned long long seq = 0) {
-  const int grid = clamp_grid(inspect_units(as.size), resident_grid(k_inspect_vc<G, F>, INSPECT_THREADS));
-  k_inspect_vc<G, F><<<grid, INSPECT_THREADS, 0, stream()>>>(as, g, f, info, skip_if, sig, seq);
+  const inspect_plan_t p = inspect_plan(as.size);
+  auto go = [&](auto parts) {
+    constexpr int P = decltype(parts)::value;
+    auto kern = k_inspect_vc<P, G, F>;
+    const int grid = p.whole ? INSPECT_NVB
+                             : clamp_grid(inspect_units(as.size), resident_grid(kern, inspect_threads(P)));
+    kern<<<grid, inspect_threads(P), 0, stream()>>>(as, g, f, info, skip_if, sig, seq);
+  };
+  if (p.parts == 4)
+    go(std::integral_constant<int, 4>{});
+  else
+    go(std::integral_constant<int, 2>{});
 }
 
 inline double now_ms() {

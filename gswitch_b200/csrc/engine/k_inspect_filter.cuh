@@ -28,18 +28,12 @@ constexpr int INSPECT_VBLOCK = 512;          // virtual threads per virtual bloc
 constexpr int INSPECT_NVB = INSPECT_VTHREADS / INSPECT_VBLOCK;
 constexpr int INSPECT_SPAN = 4;              // consecutive vertices a physical thread takes per step
 constexpr int INSPECT_OWNERS = INSPECT_VBLOCK / INSPECT_SPAN;  // 128 threads cover one virtual block
-#ifndef GSW_INSPECT_PARTS
-#define GSW_INSPECT_PARTS 2
-#endif
-constexpr int INSPECT_PARTS = GSW_INSPECT_PARTS;  // thread groups of a CTA taking alternate steps
-constexpr int INSPECT_THREADS = INSPECT_OWNERS * INSPECT_PARTS;
+// thread groups of a CTA take alternate steps: two or four of them
+constexpr int inspect_threads(int parts) { return INSPECT_OWNERS * parts; }
 constexpr int INSPECT_SCRATCH_U32 = 2 * INSPECT_VTHREADS + INSPECT_NVB;
 constexpr int INSPECT_SCRATCH_U64 = (INSPECT_SCRATCH_U32 + 1) / 2;
 #ifndef GSW_INSPECT_UNROLL
 #define GSW_INSPECT_UNROLL 2
-#endif
-#ifndef GSW_INSPECT_MINBLOCKS
-#define GSW_INSPECT_MINBLOCKS 4
 #endif
 constexpr int INSPECT_UNROLL = GSW_INSPECT_UNROLL;
 static_assert(STAT_SLOTS == 8 + 2 * INSPECT_NVB, "statistics block layout");
@@ -75,8 +69,27 @@ __host__ __device__ __forceinline__ int64_t inspect_units(int64_t n) { return (i
 // last CTA to finish only reports.  All vertex arithmetic is 32-bit (vertex
 // ids are below 2^31), and units that lie wholly below n take a path without
 // per-vertex bounds checks.
-template <typename G, typename F>
-__global__ void __launch_bounds__(INSPECT_THREADS, GSW_INSPECT_MINBLOCKS)
+// Launched with exactly INSPECT_NVB CTAs, each holds one virtual block from its
+// first step to its last and its maxima stay in the CTA: the fold through the
+// scratch (two atomics, a counter and three fences, one after the other) is what
+// a small inspection mostly takes.  inspect_plan picks the launch; device time of
+// one BFS inspection, this against one resident wave of 256-thread CTAs at every
+// size: 2^16 vertices 10.8 against 12.9 us, 2^20 12.8 against 18.8, 2^22 18.9
+// against 23.0, 2^24 39.5 against 41.4 (PageRank's, 2^22: 37 against 41.5).
+struct inspect_plan_t {
+  int parts;  // thread groups per CTA
+  bool whole;  // INSPECT_NVB CTAs, else one resident wave
+};
+inline inspect_plan_t inspect_plan(int64_t n) {
+  // below 2^19 vertices a CTA has four steps at most, two groups' worth; up to
+  // 2^24 four groups keep enough loads in flight on 256 CTAs (two groups: 2^24
+  // 49.6 us); beyond, a resident wave has more of them
+  if (n <= (int64_t)1 << 19) return {2, true};
+  if (n <= (int64_t)1 << 24) return {4, true};
+  return {2, false};
+}
+template <int INSPECT_PARTS, typename G, typename F>
+__global__ void __launch_bounds__(inspect_threads(INSPECT_PARTS), 8 / INSPECT_PARTS)
     k_inspect_vc(active_set_t as, G g, F f, unsigned long long *info, const int *skip_if = nullptr,
                  unsigned long long *sig = nullptr, unsigned long long seq = 0) {
   // captured loops: a level whose expand found an empty input ends the loop
@@ -96,8 +109,9 @@ __global__ void __launch_bounds__(INSPECT_THREADS, GSW_INSPECT_MINBLOCKS)
   const unsigned part = threadIdx.x / INSPECT_OWNERS;
   const unsigned q = threadIdx.x % INSPECT_OWNERS;
   const unsigned lane = lane_id();
+  const bool whole = gridDim.x == INSPECT_NVB;  // this CTA's units are one virtual block
   unsigned active_num = 0, inactive_num = 0;
-  unsigned long long push_wl = 0, pull_wl = 0;
+  unsigned long long push_wl = 0, pull_wl = 0, whole_p = 0, whole_l = 0;
 
   for (unsigned long long u = lo; u < hi;) {
     const unsigned b = (unsigned)(u / K);
@@ -188,6 +202,15 @@ __global__ void __launch_bounds__(INSPECT_THREADS, GSW_INSPECT_MINBLOCKS)
           s_mp[q][i] = h == 1 ? mp[i] : max(s_mp[q][i], mp[i]), s_ml[q][i] = h == 1 ? ml[i] : max(s_ml[q][i], ml[i]);
       __syncthreads();
     }
+    if (whole) {
+      if (part == 0)
+#pragma unroll
+        for (int i = 0; i < INSPECT_SPAN; ++i) {
+          whole_p += INSPECT_PARTS > 1 ? max(mp[i], s_mp[q][i]) : mp[i];
+          whole_l += INSPECT_PARTS > 1 ? max(ml[i], s_ml[q][i]) : ml[i];
+        }
+      break;
+    }
     if (part == 0) {
       unsigned *vp = vmax + b * INSPECT_VBLOCK + INSPECT_SPAN * q;
 #pragma unroll
@@ -226,20 +249,25 @@ __global__ void __launch_bounds__(INSPECT_THREADS, GSW_INSPECT_MINBLOCKS)
     u += k1 - k0;
   }
 
-  // the four counters in one block reduction
+  // the four counters, and the block's sums of maxima, in one block reduction
   {
-    unsigned long long c4[4] = {active_num, inactive_num, push_wl, pull_wl};
-    __shared__ unsigned long long s_c4[INSPECT_THREADS / 32][4];
+    unsigned long long c6[6] = {active_num, inactive_num, push_wl, pull_wl, whole_p, whole_l};
+    __shared__ unsigned long long s_c6[inspect_threads(INSPECT_PARTS) / 32][6];
+    const int nc = whole ? 6 : 4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) c4[i] = warp_sum(c4[i]);
+    for (int i = 0; i < 6; ++i)
+      if (i < nc) c6[i] = warp_sum(c6[i]);
     if (lane == 0)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) s_c4[warp_id()][i] = c4[i];
+      for (int i = 0; i < 6; ++i) s_c6[warp_id()][i] = c6[i];
     __syncthreads();
-    if (threadIdx.x < 4) {
+    if ((int)threadIdx.x < nc) {
       unsigned long long t = 0;
-      for (int w = 0; w < INSPECT_THREADS / 32; ++w) t += s_c4[w][threadIdx.x];
-      if (t) atomicAdd(info + threadIdx.x, t);
+      for (int w = 0; w < inspect_threads(INSPECT_PARTS) / 32; ++w) t += s_c6[w][threadIdx.x];
+      if (t && threadIdx.x == 4)
+        atomicMax(info + 4, t);
+      else if (t)
+        atomicAdd(info + threadIdx.x, t);
       __threadfence();
     }
     __syncthreads();
