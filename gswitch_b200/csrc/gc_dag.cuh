@@ -20,7 +20,10 @@
 // flight (a warp to a vertex took 12.5 us a level, with up to a dozen vertices
 // in turn), and the line GC_SMALL_ARCS is one such round.
 // The rows have to be sorted, so that a vertex's smaller neighbours are the
-// front of its row; the caller checks (k_row_descents).
+// front of its row; the caller checks (k_row_descents).  An undirected graph
+// also has to list each arc from both ends (k_arc_pairs): the counters come from
+// a vertex's own row and are taken down along its neighbours' rows.  Any other
+// graph keeps the level loop.
 #pragma once
 #include "engine/executor.cuh"
 

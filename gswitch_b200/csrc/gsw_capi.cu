@@ -2771,7 +2771,10 @@ gsw_status gsw_gc(gsw_ctx *ctx, gsw_graph *gr, const gsw_run_opts *o, int32_t *c
   entry_guard eg(ctx);
   if (!ctx || !gr) return fail(GSW_ERR_INVALID_ARG, "gsw_gc: bad arguments");
   begin_stats(st);
-  if (unforced(o) && rows_sorted(gr)) return gc_dag_run(ctx, gr, colors, st, eg);
+  // the counts of an undirected graph's own rows are taken back along the rows
+  // of the neighbours: both ends have to list an arc
+  if (unforced(o) && rows_sorted(gr) && (gr->directed || both_ends(ctx, gr)))
+    return gc_dag_run(ctx, gr, colors, st, eg);
   if (!ok()) return eg.finish();
   auto g = gr->view<Empty>();
   app::GC f;

@@ -1,7 +1,8 @@
 """Colouring in dependency order (k_gc_dag), the default form of Graph.gc, where
 it can go wrong: frontiers on either side of what one CTA takes, chains longer
 than one stay on a CTA, rows longer than a warp's share, duplicates, directed
-graphs, rows that are not sorted, and vertices that are their own neighbour."""
+graphs, rows that are not sorted, arcs listed from one end only, and vertices
+that are their own neighbour."""
 import numpy as np
 import pytest
 
@@ -104,4 +105,41 @@ def test_forced_and_recorded_runs_keep_the_level_loop(ctx):
     for o in ("Push-Queue-WM", "x-Bitmap", gs.RunOpts(timing=True), gs.RunOpts(persistent=False)):
         got, st = g.gc(o)
         assert np.array_equal(got, ref) and len(st.trace) == st.levels
+    g.close()
+
+
+def one_sided():
+    r = np.random.default_rng(7)
+    yield "pair", 2, np.array([0]), np.array([1])
+    yield "mixed", 6, np.array([0, 1, 2, 3, 3, 3, 4, 5]), np.array([1, 3, 0, 1, 4, 5, 3, 3])
+    for n, m in ((40, 60), (3000, 9000)):
+        u, v = r.integers(0, n, m), r.integers(0, n, m)
+        u, v = u[u != v], v[u != v]
+        yield f"up{n}", n, np.minimum(u, v), np.maximum(u, v)
+        yield f"down{n}", n, np.maximum(u, v), np.minimum(u, v)
+        yield f"some{n}", n, u, v
+        # as many arcs up as down, none listed from both ends
+        yield f"balanced{n}", n, np.concatenate([np.arange(0, n - 1, 2), np.arange(2, n, 2)]), np.concatenate(
+            [np.arange(1, n, 2), np.arange(1, n - 1, 2)])
+
+
+@pytest.mark.parametrize("case", list(one_sided()), ids=lambda c: c[0])
+def test_one_sided_arcs_keep_the_loop(ctx, case):
+    """An undirected graph that lists an arc from one end only is coloured by
+    the level loop, as it pulls and pushes along such arcs."""
+    name, n, u, v = case
+    off, col = csr(n, u, v)
+    g = ctx.upload(off, col)
+    want, ls = g.gc(gs.RunOpts(timing=True))
+    got, st = g.gc()
+    assert np.array_equal(got, want) and st.levels == ls.levels and st.trace == ls.trace
+    if name == "mixed":
+        assert got.tolist() == [4, 3, 1, 2, 1, 1]
+    g.close()
+
+
+def test_no_arcs(ctx):
+    g = ctx.upload(np.zeros(71, np.int64), np.zeros(0, np.int32))
+    got, st = g.gc()
+    assert np.array_equal(got, np.ones(70, np.int32)) and st.levels == 1
     g.close()
