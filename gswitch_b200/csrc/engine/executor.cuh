@@ -711,10 +711,17 @@ struct executor_t {
       GSW_LAUNCHED();
       all_tiles_built = PULL ? 2 : 1;
     }
-    auto kern = PULL ? k_pull_all<G, F> : k_push_all<G, F>;
     const int64_t want = (nt + ALL_WARPS - 1) / ALL_WARPS;
-    const int grid = opts().force_grid > 0 ? opts().force_grid : clamp_grid(want, resident_grid(kern, EXPAND_THREADS));
-    kern<<<grid, EXPAND_THREADS, 0, stream()>>>(as, g, f, conf, dg_all_tile, nt);
+    auto go = [&](auto kern) {
+      const int grid = opts().force_grid > 0 ? opts().force_grid : clamp_grid(want, resident_grid(kern, EXPAND_THREADS));
+      kern<<<grid, EXPAND_THREADS, 0, stream()>>>(as, g, f, conf, dg_all_tile, nt);
+    };
+    // one of the two is named: the pull stages values in shared memory, which
+    // holds 4-byte ones only
+    if constexpr (PULL)
+      go(k_pull_all<G, F>);
+    else
+      go(k_push_all<G, F>);
   }
 
   template <bool PULL, int T, typename G>
