@@ -315,7 +315,7 @@ struct inspector_t {
     // the push max counter sums per-thread maxima, so it bounds the largest
     // active degree from above; the first level has only its workload
     raw_max_push = c.max_push > 0 ? c.max_push : c.push;
-    raw_max_pull = c.max_pull > 0 ? c.max_pull : c.pull;  // likewise, summed over blocks
+    raw_max_pull = c.max_pull > 0 ? c.max_pull : c.pull;  // likewise (out-degrees), summed over blocks
   }
 
   // raw counters of the last inspection (before cross() folding)
@@ -606,7 +606,9 @@ struct executor_t {
     // grid bookkeeping of the reference (executor.cuh:30-52): idle levels
     // feed trigger_fusion, tiny STRICT levels fall back to CM
     level_grid_bookkeeping(fets, conf);
-    set_hints(as, fets, conf);
+    bool directed = false;
+    if constexpr (std::is_same<G, device_graph_t<CSR, typename G::edge_t>>::value) directed = g.directed;
+    set_hints(as, fets, conf, directed);
     if (conf.conf_centric == VC && conf.conf_fuse_inspect && !conf.conf_first_round && conf.conf_compensation &&
         as.fmt == Queue)
       compensation(as, g, f);
@@ -618,7 +620,7 @@ struct executor_t {
     fets.avg_filter_time = stat.avg_filter_time;
   }
 
-  void set_hints(active_set_t &as, const feature_t &fets, const config_t &conf) {
+  void set_hints(active_set_t &as, const feature_t &fets, const config_t &conf, bool directed) {
     hints_t &h = hints();
     if (as.fmt == Bitmap) {
       h.frontier = as.size;
@@ -639,7 +641,9 @@ struct executor_t {
                  as.fmt == Queue)
                     ? insp->raw_max_push
                     : -1;
-    if (!conf.conf_fuse_inspect && insp && conf.conf_dir == Pull && conf.conf_target == Inactive)
+    // the inspection counts out-degrees: they bound the rows a pull sweeps only
+    // where the in-rows are the same
+    if (!directed && !conf.conf_fuse_inspect && insp && conf.conf_dir == Pull && conf.conf_target == Inactive)
       h.max_deg = insp->raw_max_pull;
   }
 

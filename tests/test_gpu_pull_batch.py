@@ -1,6 +1,7 @@
 """The batched pulls and their hub pieces where they can go wrong: in-degrees on
 either side of a round, a tile, the hub lines and a hub piece, whole and divided
-vertices at the ends of a window, every mapping and STRICT tile."""
+vertices at the ends of a window, every mapping and STRICT tile; hubs of a directed
+graph, whose in-degrees no out-degree bounds."""
 import numpy as np
 import pytest
 
@@ -53,3 +54,31 @@ def test_every_pull(ctx, d):
     finally:
         ctx.tune_load_shapes(None)
         g.close()
+
+
+@pytest.mark.parametrize("lb", ["WM", "CM"])
+@pytest.mark.parametrize("d", [8191, 8192, 8193, 400000])
+def test_directed_hub(ctx, d, lb):
+    """0 -> a layer of d -> one vertex, with 3 or with 5,000 columns of its own: its
+    in-edges are spread over the CTAs whichever out-degree it has (a lone warp or
+    CTA takes 400,000 of them 30 times as long as the grid)."""
+    ms = {}
+    for own in (3, 5000):
+        a, hub = np.arange(1, d + 1), d + 1
+        u = np.concatenate([np.zeros(d, int), a, np.full(own, hub)])
+        v = np.concatenate([a, np.full(d, hub), hub + 1 + np.arange(own)])
+        h = csr(hub + 1 + own, u, v, np.ones(len(u), int))
+        lv = oracle.bfs(h, 0)
+        g = ctx.upload(h.off, h.col, directed=True)
+        cfg = f"Pull-Bitmap-{lb}-Standalone"
+        runs = []
+        for _ in range(4):
+            got, st = g.bfs(0, gs.RunOpts.from_config(cfg, timing=True))
+            assert np.array_equal(got, lv), (d, cfg, own)
+            runs.append(st.level_ms[1])  # the level that finds the hub
+        ms[own] = min(runs)
+        nsp, _, _ = g.bc(0, cfg)
+        assert np.array_equal(nsp, oracle.bc_f32(h, 0)[0]), (d, cfg, own)
+        g.close()
+    if d == 400000:
+        assert ms[3] <= 3 * ms[5000] + 0.05, ms
