@@ -1597,12 +1597,13 @@ gsw_status gsw_ctx_stream(gsw_ctx *ctx, void **s) {
 // BFS: application/bfs.cu:78-102 (loop) and :104-130 (set-up)
 // ---------------------------------------------------------------------------
 // Nothing about the level loop is asked for: no forced choice, no per-level
-// record, no per-launch form; nor, unless the caller says so, the captured one.
-static bool unforced(const gsw_run_opts *o, bool captured_too = false) {
+// record, no per-launch or captured form, no queue order, no hub sweep.  The
+// selector is no such wish: it says who picks the variants of a loop that runs.
+static bool unforced(const gsw_run_opts *o) {
   return !record_sink() && !g_label &&
-         (!o || (o->direction < 0 && o->asfmt < 0 && o->lb < 0 && o->fusion < 0 && !o->verbose && !o->timing &&
-                 o->expand_grid == 0 && !o->account && o->persistent != 0 && !o->barrier_test &&
-                 (captured_too || !o->captured)));
+         (!o || (o->direction < 0 && o->asfmt < 0 && o->lb < 0 && o->fusion < 0 && o->sorted_queue && !o->verbose &&
+                 !o->timing && o->expand_grid == 0 && !o->account && o->persistent != 0 && !o->barrier_test &&
+                 !o->captured && (o->hub_path < 0 || o->hub_path > 2)));
 }
 
 // a small graph's BFS in one launch (bfs_small.cuh): the loop's levels and
@@ -1658,8 +1659,7 @@ gsw_status bfs_run(gsw_ctx *ctx, gsw_graph *gr, const int32_t *roots, int nroots
                    int32_t *levels, gsw_run_stats *st, entry_guard &eg) {
   const int32_t root = roots[0];
   begin_stats(st);
-  // the captured form too: like the graph, the launch needs no host until the answer
-  if (unforced(o, true) && gr->n <= SB_MAX_VERTICES && gr->m <= SB_MAX_ARCS)
+  if (unforced(o) && gr->n <= SB_MAX_VERTICES && gr->m <= SB_MAX_ARCS)
     return bfs_small_run(ctx, gr, roots, nroots, levels, st, eg);
   auto g = gr->view<Empty>();
   app::BFS f;

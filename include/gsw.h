@@ -133,7 +133,13 @@ typedef struct gsw_run_opts {
   int max_iters;     /* PageRank: iterations (0 = until the eps test passes) */
   float damping;     /* PageRank damping (0.85) */
   float eps;         /* PageRank per-vertex relative change threshold */
-  int selector;      /* GSW_SELECT_RULES or GSW_SELECT_MLP */
+  int selector;      /* GSW_SELECT_RULES or GSW_SELECT_MLP: who picks the
+                        variants of a level loop.  BFS of at most 2^18 vertices
+                        and 2^22 arcs, GC and CC run no level loop unless some
+                        other field asks for one (a forced choice, unsorted
+                        queues, timing, account, verbose, persistent = 0,
+                        captured, hub_path, expand_grid) or features are
+                        recorded */
   int verbose;       /* per-level trace on stdout */
   int timing;        /* per-level device times into gsw_run_stats (CUDA
                         events around each inspect / expand, resolved after
@@ -151,9 +157,7 @@ typedef struct gsw_run_opts {
                         device-side selection and termination (BFS, SSSP, PR,
                         delta-PR, CC, GC; GSW_ERR_UNSUPPORTED for BC, MBFS and
                         batched BC, whose batched forms run every level in one
-                        cooperative launch; a small graph's BFS with no forced
-                        choice is one such launch in either form); 0:
-                        host-driven loop */
+                        cooperative launch); 0: host-driven loop */
   int hub_path;      /* how a CTA sweeps one hub's adjacency list (the
                         thread/warp/CTA-tiered push's CTA tier): 0 four-byte
                         loads, 1 int4 loads of the 16-byte-aligned body,

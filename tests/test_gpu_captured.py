@@ -83,7 +83,7 @@ def test_captured_persistent_fused_levels(ctx, graphs, name):
     g = ctx.upload(h.off, h.col)
     ref = oracle.bfs(h, root)
     for cfg in ["", "Push-Queue-WM-Fused", "Push-Queue-STRICT-Fused", "Push-Queue-TWC-Fused", "Push-Queue-CM-Fused"]:
-        _, host = g.bfs(root, gs.RunOpts.from_config(cfg))
+        _, host = g.bfs(root, gs.RunOpts.from_config(cfg, timing=True))  # timed: the loop on a small graph too
         for _ in range(2):
             lv, st = g.bfs(root, cap(cfg))
             assert np.array_equal(lv, ref), (name, cfg)

@@ -102,7 +102,8 @@ def test_forced_and_recorded_runs_keep_the_level_loop(ctx):
     h = oracle.rmat(10, 8, seed=2)
     g = ctx.upload(h.off, h.col)
     ref = oracle.gc_levels(h)
-    for o in ("Push-Queue-WM", "x-Bitmap", gs.RunOpts(timing=True), gs.RunOpts(persistent=False)):
+    for o in ("Push-Queue-WM", "x-Bitmap", gs.RunOpts(timing=True), gs.RunOpts(persistent=False),
+              gs.RunOpts(sorted_queue=False), gs.RunOpts(hub_path=0)):
         got, st = g.gc(o)
         assert np.array_equal(got, ref) and len(st.trace) == st.levels
     g.close()

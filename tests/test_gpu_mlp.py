@@ -151,8 +151,9 @@ def test_results_exact_under_network_choices(ctx):
     for s in range(4):
         ctx.mlp_load(random_model(rng), 0.0)
         for captured in (False, True):
-            lv, _ = g.bfs(root, gs.RunOpts(selector="mlp", captured=captured))
-            assert np.array_equal(lv, ref_bfs), (s, captured)
+            # timed: the loop on a small graph too
+            lv, st = g.bfs(root, gs.RunOpts(selector="mlp", captured=captured, timing=not captured))
+            assert np.array_equal(lv, ref_bfs) and len(st.trace) > 1, (s, captured)
         d, _ = g.sssp(root, gs.RunOpts(selector="mlp"))
         assert np.array_equal(d, ref_sssp), s
     ctx.mlp_load(None)

@@ -35,7 +35,7 @@ def test_results_exact_under_extreme_grids(ctx, quarters):
         dref = oracle.sssp_dijkstra(hw, root)
         for cfg in ["", "Push-Queue-WM", "Push-Queue-STRICT-Fused", "Pull-Bitmap-TM", "Push-Bitmap-TWC",
                     "Pull-Queue-CM"]:
-            lv, _ = g.bfs(root, cfg)
+            lv, _ = g.bfs(root, gs.RunOpts.from_config(cfg, timing=True))  # timed: the loop on a small graph too
             assert np.array_equal(lv, ref), (quarters, cfg)
             d, _ = g.sssp(root, cfg)
             assert np.array_equal(d, dref), (quarters, cfg)
