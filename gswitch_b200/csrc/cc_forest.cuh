@@ -12,9 +12,14 @@
 // (provided that each arc is listed from both ends, which k_arc_pairs checks).
 // Hooking always puts the larger root under the smaller one, so a component's
 // label is its smallest vertex, as in the loop.
-// What bounds it: eight short passes over the vertices, each with a random
-// label read per vertex: 207 us of kernels on RMAT 2^22, where the loop's two
-// inspections, two hooking passes and pointer jumps took 1,183 us.
+// The trees are flattened before every pass that climbs them: ids that follow a
+// path or a mesh make the first trees as deep as the graph is long, and hooking
+// climbs one vertex at a time (two interleaved paths of 2^20 vertices: 0.08 ms,
+// 89 ms with one flatten before the last pass).
+// What bounds it: ten short passes over the vertices, each with a random label
+// read per vertex: 176 us on RMAT 2^22, where the loop's two inspections, two
+// hooking passes and pointer jumps took 1,183 us (207 us with one flatten: the
+// hooking passes climbed the difference).
 #pragma once
 #include "engine/executor.cuh"
 #include "graphgen.cuh"
@@ -72,12 +77,13 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_link_one(const int64_t *off, 
     else if (e - b == 1) cc_link(comp, (int)v, __ldg(col + b));
   }
 }
+// every vertex under its root (roots stay roots meanwhile).  Each step is
+// written at once: threads further down the same chain then jump over what this
+// one has climbed, and a chain of n vertices takes log n steps and not n.
 __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *comp, int64_t n) {
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-    const int p0 = comp[v];
-    int p = p0, q;
-    while (p != (q = comp[p])) p = q;  // roots stay roots meanwhile
-    if (p != p0) comp[v] = p;
+    int p = comp[v], q;
+    while (p != (q = comp[p])) comp[v] = p = q;
   }
 }
 // the most common label among CC_SAMPLE vertices spread over the ids

@@ -2240,7 +2240,10 @@ static gsw_status cc_forest_run(gsw_ctx *ctx, gsw_graph *gr, int32_t *labels, gs
   timer tm(ctx);
   k_cc_start<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp);
   GSW_LAUNCHED();
+  // flat trees before every pass that climbs them (cc_link takes a step at a time)
   for (int last = 0; last < 2; ++last) {
+    k_cc_flatten<<<grid, CC_THREADS, 0, stream()>>>(comp, n);
+    GSW_LAUNCHED();
     k_cc_link_one<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp, last != 0);
     GSW_LAUNCHED();
   }

@@ -1,7 +1,7 @@
 """Components by sampled hooking (the default form of Graph.cc) where it can go
 wrong: rows on either side of what a lane, a warp and a piece take, hubs outside
-the most common component, chains, many equal components, graphs that list each
-edge once, directed graphs, self-loops and duplicates."""
+the most common component, chains (also in id order), many equal components,
+graphs that list each edge once, directed graphs, self-loops and duplicates."""
 import numpy as np
 import pytest
 
@@ -83,4 +83,29 @@ def test_one_sided_arcs_keep_the_loop(ctx):
     g = ctx.upload(off, col)
     want = g.cc("x-Bitmap")[0]
     assert np.array_equal(g.cc()[0], want)
+    g.close()
+
+
+def chains():
+    n = 1 << 18
+    yield "path", n, np.arange(n - 1), np.arange(1, n)
+    # two paths, of the even and the odd ids, joined where both end
+    yield "interleaved", n, np.concatenate([np.arange(n - 2), [n - 2]]), np.concatenate([np.arange(2, n), [n - 1]])
+    at = np.arange(n).reshape(n // 4, 4)
+    yield "strip", n, np.concatenate([at[:-1].ravel(), at[:, :-1].ravel()]), np.concatenate(
+        [at[1:].ravel(), at[:, 1:].ravel()])
+
+
+@pytest.mark.parametrize("case", list(chains()), ids=lambda c: c[0])
+def test_chains_in_id_order(ctx, case):
+    """Trees as deep as the graph is long (ids along a path or a mesh) are
+    flattened before anything climbs them: the time stays near the loop's, where
+    a climb of one vertex at a time takes a hundred times as long."""
+    name, n, u, v = case
+    off, col = csr(n, np.concatenate([u, v]), np.concatenate([v, u]))
+    g = ctx.upload(off, col)
+    loop = min(g.cc("x-Bitmap", out=False)[1].ms for _ in range(4))
+    runs = [g.cc() for _ in range(4)]
+    assert all(not lab.any() for lab, _ in runs)  # one component
+    assert min(st.ms for _, st in runs) <= 4 * loop + 0.2, (loop, [st.ms for _, st in runs])
     g.close()
