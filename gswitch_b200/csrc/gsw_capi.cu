@@ -2728,8 +2728,9 @@ static gsw_status gc_dag_run(gsw_ctx *ctx, gsw_graph *gr, int32_t *colors, gsw_r
   const size_t row = sizeof(int) * (gr->n + 1);
   int *wait = (int *)ctx->buf("wa", row), *colour = (int *)ctx->buf("ra", row), *low = (int *)ctx->buf("gc_low", row);
   int *q0 = (int *)ctx->buf("gc_q0", row), *q1 = (int *)ctx->buf("gc_q1", row);
+  gc_piece_t *piece = (gc_piece_t *)ctx->buf("gc_pieces", sizeof(gc_piece_t) * gc_pieces(gr->m));
   gc_state_t *S = (gc_state_t *)ctx->buf("gc_state", sizeof(gc_state_t));
-  if (!wait || !colour || !low || !q0 || !q1 || !S) return eg.finish();
+  if (!wait || !colour || !low || !q0 || !q1 || !piece || !S) return eg.finish();
   auto g = gr->view<Empty>();
   unsigned long long budget = 2000000000ull;  // per barrier wait
   // one warp per 32 vertices fills the grid; a small graph takes fewer CTAs
@@ -2740,7 +2741,7 @@ static gsw_status gc_dag_run(gsw_ctx *ctx, gsw_graph *gr, int32_t *colors, gsw_r
   for (int first = 1; ok(); first = 0) {
     if (!first) GSW_CUDA(cudaMemsetAsync(S, 0, offsetof(gc_state_t, pub), stream()));
     void *args[] = {(void *)&g,  (void *)&wait, (void *)&low, (void *)&colour, (void *)&q0,
-                    (void *)&q1, (void *)&S,    (void *)&first, (void *)&budget};
+                    (void *)&q1, (void *)&piece, (void *)&S, (void *)&first, (void *)&budget};
     if (GSW_CUDA(cudaLaunchCooperativeKernel((const void *)k_gc_dag, grid, GC_THREADS, args, 0, stream()))) break;
     GSW_LAUNCHED();
     GSW_CUDA(cudaMemcpyAsync(&h, S, sizeof(h), cudaMemcpyDeviceToHost, stream()));

@@ -40,6 +40,19 @@ def both(u, v):
     return np.concatenate([u, v]), np.concatenate([v, u])
 
 
+def hubs(sizes, k, late):
+    """One vertex above d leaves for each d of sizes, k pairs; late: the hubs wait for
+    one vertex, the pairs' larger ends for k others."""
+    leaves, at = int(sum(sizes)), np.cumsum([0] + sizes)
+    top = leaves + k + np.arange(len(sizes) + k)  # hubs, then the pairs' larger ends
+    u = np.concatenate([np.repeat(top[:len(sizes)], sizes), top[len(sizes):]])
+    v = np.concatenate([np.arange(leaves), leaves + np.arange(k)])
+    if late:
+        above = top[-1] + 1 + np.concatenate([np.zeros(len(sizes), int), 1 + np.arange(k)])
+        u, v = np.concatenate([u, above]), np.concatenate([v, top])
+    return u, v
+
+
 def graphs():
     r = np.random.default_rng(3)
     for n in (1, 2, 33, 5000):  # a chain of n levels
@@ -47,6 +60,11 @@ def graphs():
     for n in (1023, 1025, 3000):  # frontiers of n - 1 vertices around one hub, smallest or largest
         yield f"star_low{n}", n, np.zeros(n - 1, int), np.arange(1, n)
         yield f"star_high{n}", n, np.full(n - 1, n - 1), np.arange(n - 1)
+    # rows on either side of what a warp takes and of a piece, in frontiers of fewer
+    # and of more vertices than the grid has warps, found by CTA 0 and by the grid
+    for k, late in ((3, 0), (3, 1), (3000, 0), (6000, 0), (6000, 1)):
+        u, v = hubs([255, 256, 1023, 1024, 1025, 1279, 1281, 8191, 8193, 30000], k, late)
+        yield f"hubs{k}_{late}", int(max(u.max(), v.max())) + 1, u, v
     yield "clique", 300, *np.nonzero(np.triu(np.ones((300, 300), int), 1))
     yield "layers", 9000, np.repeat(np.arange(6000), 3), np.minimum(np.repeat(np.arange(6000), 3) + 3000 * (
         1 + np.arange(18000) % 2) // 2 + r.integers(0, 900, 18000), 8999)
@@ -143,4 +161,24 @@ def test_no_arcs(ctx):
     g = ctx.upload(np.zeros(71, np.int64), np.zeros(0, np.int32))
     got, st = g.gc()
     assert np.array_equal(got, np.ones(70, np.int32)) and st.levels == 1
+    g.close()
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("late", [0, 1])
+def test_long_rows_are_spread(ctx, directed, late):
+    """A row of 2^18 smaller neighbours in a frontier of more vertices than the grid
+    has warps takes no longer than the loop's sweeps (a lone warp: 7 ms)."""
+    u, v = hubs([1 << 18], 6000, late)
+    n = int(u.max()) + 1
+    ref = colours(n, u, v)
+    off, col = csr(n, u, v) if directed else csr(n, *both(u, v))
+    g = ctx.upload(off, col, directed=directed)
+    ms = []
+    for _ in range(4):
+        got, st = g.gc()
+        assert np.array_equal(got, ref)
+        ms.append(st.ms)
+    loop = min(g.gc(gs.RunOpts(timing=True))[1].ms for _ in range(4))
+    assert min(ms) <= 2 * loop + 0.3, (ms, loop)
     g.close()
