@@ -466,8 +466,12 @@ __device__ __forceinline__ void pull_edges(const active_set_t &as, const G &g, F
 // true there if the run has a message.  Every lane of the warp calls it.
 template <typename WA, typename G, typename F>
 __device__ __forceinline__ bool fold_runs(F &f, const G &g, int id, bool have, WA &io) {
-  // by value: clearing the array of messages with memset and folding in place,
-  // nvcc 12.9 lost updates of a mixed int/float message (BCBackward)
+  // By value, of value-initialised messages: with the messages cleared by memset
+  // and folded in place, nvcc 12.9 loses updates where comp changes one word of a
+  // two-word message.  A kernel of this fold alone shows it: wrong sums at its
+  // optimiser's -O3, right ones at that optimiser's -O1 whatever ptxas' level.
+  // Functors that sum every word or one word of theirs are run under every variant
+  // by the tests.
   WA x = io;
   const int lane = lane_id();
 #pragma unroll
