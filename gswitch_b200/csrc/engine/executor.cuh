@@ -836,8 +836,10 @@ struct executor_t {
         }
         case STRICT: {
           // every vertex sends along all of its out-edges: no scan (the same
-          // line as for the pull below)
-          if (!fused && conf.conf_fromall && conf.conf_toall && !conf.conf_fixed && as.fmt == Bitmap) {
+          // line as for the pull below; a pruned push keeps a target's first
+          // message only, which the scanned form looks after)
+          if (!fused && conf.conf_fromall && conf.conf_toall && !conf.conf_fixed && !conf.conf_pruning &&
+              as.fmt == Bitmap) {
             launch_all<false>(as, g, f, conf);
             break;
           }

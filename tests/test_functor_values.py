@@ -110,3 +110,16 @@ def test_every_variant_sums_every_word(built, words, one, directed):
                 if f == "Bitmap":
                     got = level(L, words, n, u, v, directed, active, x, (d, f, lb), everything=1)
                     assert np.array_equal(got, ref_all), (d, f, lb, "all")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lb", ["TM", "WM", "CM", "STRICT", "TWC"])
+def test_pruned_push_delivers_to_a_target_once(built, lb):
+    """conf_pruning: a target that has been sent to takes nothing in later levels, also
+    where every vertex sends to every vertex."""
+    n, u, v = graph("out")
+    x = np.ones(n, value_type(1))
+    indeg = np.bincount(v, minlength=n)
+    got = level(built[1, 0], 1, n, u, v, "out", np.ones(n, np.int32), x, ("Push", "Bitmap", lb), everything=1, pruning=1,
+                passes=2)["a"][:, 0]
+    assert np.array_equal(got > 0, indeg > 0) and (got <= indeg).all()
