@@ -32,10 +32,13 @@ constexpr int CC_ROW_PIECE = 4096;  // and from which it is cut for several warp
 constexpr int CC_SAMPLE = 1024;
 
 struct cc_state_t {
-  unsigned long long up;      // arcs v -> u with u > v (the undirected edges)
+  int common;  // the most common label
+  int pieces;  // listed row pieces
+};
+struct row_facts_t {
+  unsigned long long up;       // arcs v -> u with u > v (the undirected edges)
   unsigned long long balance;  // sum over arcs of +-hash(smaller, larger): 0 when each is listed from both ends
-  int common;                 // the most common label
-  int pieces;                 // listed row pieces
+  long long descents;          // inside rows (k_row_descents): 0 when every row ascends
 };
 struct cc_piece_t {
   int64_t beg;
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_pieces(const int *col, int *c
 // Also counts the edges.  One warp per 256 slots of the rows, as the all-to-all
 // expands lay them out.
 __global__ void __launch_bounds__(EXPAND_THREADS) k_arc_pairs(const int64_t *off, const int *col, int64_t n, int64_t m,
-                                                              const int *tile_lo, int64_t ntiles, cc_state_t *S) {
+                                                              const int *tile_lo, int64_t ntiles, row_facts_t *F) {
   __shared__ unsigned short s_begs[ALL_WARPS][ALL_TILE + 2];
   const int lane = lane_id();
   unsigned short *s_beg = s_begs[warp_id()];
@@ -193,8 +196,8 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_arc_pairs(const int64_t *off
   up = warp_sum(up);
   balance = warp_sum(balance);
   if (lane == 0) {
-    atomicAdd(&S->up, up);
-    atomicAdd(&S->balance, balance);
+    atomicAdd(&F->up, up);
+    atomicAdd(&F->balance, balance);
   }
 }
 

@@ -2206,27 +2206,38 @@ static bool cc_captured_run(gsw_ctx *ctx, device_graph_t<COO, Empty> g, app::CC 
   return ok();
 }
 
-// is the graph stored with every arc listed from both ends? (an undirected
-// upload that lists each edge once is taken as it is by the edge-centric loop)
-static bool both_ends(gsw_ctx *ctx, gsw_graph *g) {
-  if (g->both_ends < 0) {
-    executor_t &ex = ctx->executor;
-    cc_state_t *S = (cc_state_t *)ctx->buf("cc_state", sizeof(cc_state_t)), h{};
-    ex.ensure_all_tiles(g->n, g->m);
-    if (!S || !ok()) return false;
+// Looks once at what a graph's rows are, both facts with one wait: whether every
+// adjacency ascends, and whether every arc is listed from both ends (an undirected
+// upload that lists each edge once is taken as it is by the level loops).
+static bool look_at_rows(gsw_ctx *ctx, gsw_graph *g, bool sorted, bool ends) {
+  sorted = sorted && g->rows_sorted < 0;
+  ends = ends && g->both_ends < 0;
+  if (!sorted && !ends) return true;
+  executor_t &ex = ctx->executor;
+  row_facts_t *F = (row_facts_t *)ctx->buf("row_facts", sizeof(row_facts_t)), h{};
+  if (ends) ex.ensure_all_tiles(g->n, g->m);
+  if (!F || !ok()) return false;
+  GSW_CUDA(cudaMemsetAsync(F, 0, sizeof(row_facts_t), stream()));
+  if (sorted) {
+    k_row_descents<<<grid_for(g->m), 256, 0, stream()>>>(g->off, g->col, g->n, g->m, &F->descents);
+    GSW_LAUNCHED();
+  }
+  if (ends) {
     const int64_t nt = executor_t::all_tiles(g->n, g->m);
-    GSW_CUDA(cudaMemsetAsync(S, 0, sizeof(cc_state_t), stream()));
     k_all_tiles<<<clamp_grid((nt + 255) / 256, sm_count() * 8), 256, 0, stream()>>>(g->off, g->n, nt, ex.dg_all_tile);
     k_arc_pairs<<<clamp_grid((nt + ALL_WARPS - 1) / ALL_WARPS, resident_grid(k_arc_pairs, EXPAND_THREADS)),
-                  EXPAND_THREADS, 0, stream()>>>(g->off, g->col, g->n, g->m, ex.dg_all_tile, nt, S);
+                  EXPAND_THREADS, 0, stream()>>>(g->off, g->col, g->n, g->m, ex.dg_all_tile, nt, F);
     GSW_LAUNCHED();
-    GSW_CUDA(cudaMemcpyAsync(&h, S, sizeof(h), cudaMemcpyDeviceToHost, stream()));
-    GSW_CUDA(cudaStreamSynchronize(stream()));
-    if (!ok()) return false;
+  }
+  GSW_CUDA(cudaMemcpyAsync(&h, F, sizeof(h), cudaMemcpyDeviceToHost, stream()));
+  GSW_CUDA(cudaStreamSynchronize(stream()));
+  if (!ok()) return false;
+  if (sorted) g->rows_sorted = h.descents == 0;
+  if (ends) {
     g->both_ends = h.balance == 0;
     g->up_arcs = (int64_t)h.up;
   }
-  return g->both_ends == 1;
+  return true;
 }
 
 // components by sampled hooking (cc_forest.cuh): the loop's labels
@@ -2278,7 +2289,8 @@ gsw_status gsw_cc(gsw_ctx *ctx, gsw_graph *gr, const gsw_run_opts *o, int32_t *l
   entry_guard eg(ctx);
   if (!ctx || !gr) return fail(GSW_ERR_INVALID_ARG, "gsw_cc: bad arguments");
   begin_stats(st);
-  if (unforced(o) && !gr->directed && gr->m > 0 && both_ends(ctx, gr) && gr->up_arcs > 0)
+  if (unforced(o) && !gr->directed && gr->m > 0 && look_at_rows(ctx, gr, false, true) && gr->both_ends == 1 &&
+      gr->up_arcs > 0)
     return cc_forest_run(ctx, gr, labels, st, eg);
   if (!ok()) return eg.finish();
   if (ensure_coo(gr)) return eg.finish();
@@ -2709,20 +2721,6 @@ gsw_status gsw_bc(gsw_ctx *ctx, gsw_graph *gr, int32_t root, const gsw_run_opts 
 // ---------------------------------------------------------------------------
 // GC: application/gc.cu:76-99 (loop) and :101-122 (set-up)
 // ---------------------------------------------------------------------------
-static bool rows_sorted(gsw_graph *g) {
-  if (g->rows_sorted < 0) {
-    long long *d = (long long *)g->ctx->buf("row_descents", sizeof(long long)), h = 1;
-    if (!d) return false;
-    GSW_CUDA(cudaMemsetAsync(d, 0, sizeof(long long), stream()));
-    k_row_descents<<<grid_for(g->m), 256, 0, stream()>>>(g->off, g->col, g->n, g->m, d);
-    GSW_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, stream()));
-    GSW_CUDA(cudaStreamSynchronize(stream()));
-    if (!ok()) return false;
-    g->rows_sorted = h == 0;
-  }
-  return g->rows_sorted == 1;
-}
-
 // the colouring in dependency order (gc_dag.cuh): the level loop's colours
 static gsw_status gc_dag_run(gsw_ctx *ctx, gsw_graph *gr, int32_t *colors, gsw_run_stats *st, entry_guard &eg) {
   const size_t row = sizeof(int) * (gr->n + 1);
@@ -2777,7 +2775,8 @@ gsw_status gsw_gc(gsw_ctx *ctx, gsw_graph *gr, const gsw_run_opts *o, int32_t *c
   begin_stats(st);
   // the counts of an undirected graph's own rows are taken back along the rows
   // of the neighbours: both ends have to list an arc
-  if (unforced(o) && rows_sorted(gr) && (gr->directed || both_ends(ctx, gr)))
+  if (unforced(o) && look_at_rows(ctx, gr, true, !gr->directed) && gr->rows_sorted == 1 &&
+      (gr->directed || gr->both_ends == 1))
     return gc_dag_run(ctx, gr, colors, st, eg);
   if (!ok()) return eg.finish();
   auto g = gr->view<Empty>();
