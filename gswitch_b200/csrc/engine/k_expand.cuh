@@ -462,10 +462,15 @@ __device__ __forceinline__ void pull_edges(const active_set_t &as, const G &g, F
     x[k] = have[k] ? f.emit(u[k], g.fetch_edata_r(ei[k]), g) : typename F::wa_t();
 }
 
-// Folds the messages of each run of lanes with the same id into its first lane;
-// true there if the run has a message.  Every lane of the warp calls it.
+// Is this lane the first of a run of lanes with the same id?
+__device__ __forceinline__ bool run_head(int id) {
+  const int pid = __shfl_up_sync(FULL, id, 1);
+  return lane_id() == 0 || pid != id;
+}
+// Folds the messages of each run of lanes with the same id into its first lane
+// (head); true there if the run has a message.  Every lane of the warp calls it.
 template <typename WA, typename G, typename F>
-__device__ __forceinline__ bool fold_runs(F &f, const G &g, int id, bool have, WA &io) {
+__device__ __forceinline__ bool fold_runs(F &f, const G &g, int id, bool head, bool have, WA &io) {
   // By value, of value-initialised messages: with the messages cleared by memset
   // and folded in place, nvcc 12.9 loses updates where comp changes one word of a
   // two-word message.  A kernel of this fold alone shows it: wrong sums at its
@@ -488,8 +493,11 @@ __device__ __forceinline__ bool fold_runs(F &f, const G &g, int id, bool have, W
     }
   }
   io = x;
-  const int pid = __shfl_up_sync(FULL, id, 1);
-  return have && (lane == 0 || pid != id);
+  return have && head;
+}
+template <typename WA, typename G, typename F>
+__device__ __forceinline__ bool fold_runs(F &f, const G &g, int id, bool have, WA &io) {
+  return fold_runs(f, g, id, run_head(id), have, io);
 }
 
 template <typename G, typename F>
@@ -612,7 +620,12 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_push_cm(active_set_t as, G g
 
 // The messages of a warp's 32 edges meet in registers first: with an atomic an
 // edge, a hub's all went to one address (4.2 ms for one backward level of
-// betweenness on RMAT 2^20).
+// betweenness on RMAT 2^20).  Up to CM_FOLD_MIN messages a vertex an atomic each
+// costs less than the fold, five PageRank iterations and a BFS forced to this pull:
+// G(2^20, 2^21) 0.30 and 0.64 against 0.35 and 0.73 ms, lattice of 2^20 0.25 and
+// 1.80 against 0.31 and 1.98 ms; RMAT 2^20, whose hubs fold, 6.9 and 3.3 against
+// 6.6 and 3.3 ms (20.6 and 9.6 ms with an atomic an edge).
+constexpr int CM_FOLD_MIN = 4;
 template <typename G, typename F>
 __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_cm(active_set_t as, G g, F f, config_t conf,
                                                             hub_list_t hubs) {
@@ -659,8 +672,12 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_pull_cm(active_set_t as, G g
       pull_edges(as, g, f, conf, u, ei, have, x);
 #pragma unroll
       for (int k = 0; k < EDGE_BATCH; ++k) {
-        if (!__any_sync(FULL, have[k])) continue;
-        if (fold_runs(f, g, id[k], have[k], x[k])) f.compAtomic(f.wa_of(s_v[id[k]]), x[k], g);
+        const unsigned sent = __ballot_sync(FULL, have[k]);
+        if (!sent) continue;
+        const bool head = run_head(id[k]);
+        const bool fold = __popc(sent) > CM_FOLD_MIN * __popc(__ballot_sync(FULL, head));
+        const bool mine = fold ? fold_runs(f, g, id[k], head, have[k], x[k]) : have[k];
+        if (mine) f.compAtomic(f.wa_of(s_v[id[k]]), x[k], g);
       }
     }
     __syncthreads();

@@ -123,3 +123,24 @@ def test_pruned_push_delivers_to_a_target_once(built, lb):
     got = level(built[1, 0], 1, n, u, v, "out", np.ones(n, np.int32), x, ("Push", "Bitmap", lb), everything=1, pruning=1,
                 passes=2)["a"][:, 0]
     assert np.array_equal(got > 0, indeg > 0) and (got <= indeg).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("degree", [1, 2, 3, 4, 5, 31, 33, 300])
+def test_pulls_of_few_messages_and_of_many_vertices(built, degree):
+    """A CTA-mapped pull sends a warp's messages on one by one where they are few, or of
+    many vertices, and folds them otherwise: on either side of both lines."""
+    r = np.random.default_rng(degree)
+    targets = 1500
+    deg = r.integers(max(1, degree - 1), degree + 2, targets)
+    v = np.repeat(np.arange(targets), deg)
+    u = targets + r.integers(0, 5000, len(v))
+    n = targets + 5000
+    x = values(2, n, r)
+    for share in (0.03, 0.22, 0.25, 0.28, 1.0):
+        active = np.concatenate([np.zeros(targets, int), r.random(5000) < share]).astype(np.int32)
+        sent = active[u] == 1
+        ref = sums_of(n, u[sent], v[sent], x)
+        for lb in ("WM", "CM"):
+            got = level(built[2, 0], 2, n, u, v, "out", active, x, ("Pull", "Bitmap", lb))
+            assert np.array_equal(got, ref), (share, lb)
