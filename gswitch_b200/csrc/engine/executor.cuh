@@ -607,8 +607,10 @@ struct executor_t {
     // feed trigger_fusion, tiny STRICT levels fall back to CM
     level_grid_bookkeeping(fets, conf);
     bool directed = false;
-    if constexpr (std::is_same<G, device_graph_t<CSR, typename G::edge_t>>::value) directed = g.directed;
-    set_hints(as, fets, conf, directed);
+    int64_t max_in = -1;
+    if constexpr (std::is_same<G, device_graph_t<CSR, typename G::edge_t>>::value)
+      directed = g.directed, max_in = g.max_in_degree;
+    set_hints(as, fets, conf, directed, max_in);
     if (conf.conf_centric == VC && conf.conf_fuse_inspect && !conf.conf_first_round && conf.conf_compensation &&
         as.fmt == Queue)
       compensation(as, g, f);
@@ -620,7 +622,7 @@ struct executor_t {
     fets.avg_filter_time = stat.avg_filter_time;
   }
 
-  void set_hints(active_set_t &as, const feature_t &fets, const config_t &conf, bool directed) {
+  void set_hints(active_set_t &as, const feature_t &fets, const config_t &conf, bool directed, int64_t max_in) {
     hints_t &h = hints();
     if (as.fmt == Bitmap) {
       h.frontier = as.size;
@@ -642,9 +644,13 @@ struct executor_t {
                     ? insp->raw_max_push
                     : -1;
     // the inspection counts out-degrees: they bound the rows a pull sweeps only
-    // where the in-rows are the same
-    if (!directed && !conf.conf_fuse_inspect && insp && conf.conf_dir == Pull && conf.conf_target == Inactive)
-      h.max_deg = insp->raw_max_pull;
+    // where the in-rows are the same; the graph's own largest in-degree always does
+    if (conf.conf_dir == Pull) {
+      h.max_deg = max_in;
+      if (!directed && !conf.conf_fuse_inspect && insp && conf.conf_target == Inactive &&
+          (h.max_deg < 0 || insp->raw_max_pull < h.max_deg))
+        h.max_deg = insp->raw_max_pull;
+    }
   }
 
   // deferred filter updates of fused levels (kernel_fusion.cuh:54-109)

@@ -30,6 +30,7 @@ struct device_graph_t<CSR, E> {
   int64_t nedges;
   int level;
   bool directed;
+  int max_in_degree = -1;  // the longest in-row, where known
   // captured level loops keep the level in device memory (the loop advances
   // it between levels); null: the by-value member above
   const int *dlevel = nullptr;

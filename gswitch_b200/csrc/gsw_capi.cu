@@ -44,6 +44,7 @@ struct gsw_graph {
   int64_t ncoo = -1;
   double attr[6] = {0, 0, 0, 0, 0, 0};
   double mean_weight = 0;
+  int max_in_degree = -1;  // the longest in-row
   int both_ends = -1;     // every arc is listed from both ends (-1: not looked at yet)
   int64_t up_arcs = -1;   // arcs v -> u with u > v, counted with it
   int rows_sorted = -1;   // every adjacency ascends (-1: not looked at yet)
@@ -72,6 +73,7 @@ struct gsw_graph {
     g.nedges = m;
     g.level = 0;
     g.directed = directed;
+    g.max_in_degree = max_in_degree;
     return g;
   }
 };
@@ -303,6 +305,7 @@ void compute_attr(gsw_graph *g) {
   g->attr[1] = sd;
   g->attr[2] = (double)(mx - (mn < 0 ? 0 : mn));
   g->attr[3] = mx;
+  if (!g->directed) g->max_in_degree = mx;
   g->attr[4] = gi;
   g->attr[5] = her;
 }
@@ -1335,7 +1338,12 @@ gsw_status gsw_graph_upload(gsw_ctx *ctx, int64_t n, int64_t m, const int64_t *r
   if (okk && g->directed) {
     std::vector<int64_t> roff(n + 1, 0);
     for (int64_t e = 0; e < m; ++e) roff[(size_t)col[e] + 1]++;
-    for (int64_t v = 0; v < n; ++v) roff[v + 1] += roff[v];
+    int64_t max_in = 0;
+    for (int64_t v = 0; v < n; ++v) {
+      max_in = std::max(max_in, roff[v + 1]);
+      roff[v + 1] += roff[v];
+    }
+    g->max_in_degree = (int)std::min(max_in, (int64_t)INT_MAX);
     std::vector<int> rcol(m), rw(weights ? m : 0);
     std::vector<int64_t> fillp(roff.begin(), roff.end() - 1);
     for (int64_t v = 0; v < n; ++v)
