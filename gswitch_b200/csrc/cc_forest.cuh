@@ -17,9 +17,8 @@
 // climbs one vertex at a time (two interleaved paths of 2^20 vertices: 0.08 ms,
 // 89 ms with one flatten before the last pass).
 // What bounds it: ten short passes over the vertices, each with a random label
-// read per vertex: 176 us on RMAT 2^22, where the loop's two inspections, two
-// hooking passes and pointer jumps took 1,183 us (207 us with one flatten: the
-// hooking passes climbed the difference).
+// read per vertex: 158 us on RMAT 2^22, where the loop's two inspections, two
+// hooking passes and pointer jumps took 1,183 us.
 #pragma once
 #include "engine/executor.cuh"
 #include "graphgen.cuh"
@@ -45,6 +44,28 @@ struct cc_piece_t {
   int v, len;
 };
 
+// The passes are short, so each is set up while the one before still runs
+// (programmatic dependent launch: the next may be launched at once, and waits here
+// for everything the one before writes).  With ten passes a call on RMAT 2^16 takes
+// 50 us, 69 us with plain launches (61 us with eight); 2^22 179 and 194 us.
+__device__ __forceinline__ void cc_begin() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+template <typename... P, typename... A>
+inline void cc_launch(void (*kern)(P...), int grid, int threads, bool first, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = stream();
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = first ? 0 : 1;  // whatever ran before the first pass ends before it
+  if (!GSW_CUDA(cudaLaunchKernelEx(&cfg, kern, P(args)...))) GSW_LAUNCHED();
+}
+
 // Joins the trees of u and v: the larger root goes under the smaller.  Labels
 // are read through the L1: an old label is still an ancestor (labels only move
 // towards the root), and the root that all of a large component reads would
@@ -66,6 +87,7 @@ __device__ __forceinline__ void cc_link(int *comp, int u, int v) {
 // every vertex under its first neighbour where that is the smaller: a forest,
 // since parents only get smaller
 __global__ void __launch_bounds__(CC_THREADS) k_cc_start(const int64_t *off, const int *col, int64_t n, int *comp) {
+  cc_begin();
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = __ldg(off + v), e = __ldg(off + v + 1);
     comp[v] = b < e ? min((int)v, __ldg(col + b)) : (int)v;
@@ -74,6 +96,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_start(const int64_t *off, con
 // along the second arc, or the last
 __global__ void __launch_bounds__(CC_THREADS) k_cc_link_one(const int64_t *off, const int *col, int64_t n, int *comp,
                                                             bool last) {
+  cc_begin();
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = __ldg(off + v), e = __ldg(off + v + 1);
     if (e - b > (last ? 2 : 1)) cc_link(comp, (int)v, __ldg(col + (last ? e - 1 : b + 1)));
@@ -84,6 +107,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_link_one(const int64_t *off, 
 // written at once: threads further down the same chain then jump over what this
 // one has climbed, and a chain of n vertices takes log n steps and not n.
 __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *comp, int64_t n) {
+  cc_begin();
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
     int p = comp[v], q;
     while (p != (q = comp[p])) comp[v] = p = q;
@@ -91,6 +115,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *comp, int64_t n)
 }
 // the most common label among CC_SAMPLE vertices spread over the ids
 __global__ void __launch_bounds__(CC_SAMPLE) k_cc_common(const int *comp, int64_t n, cc_state_t *S) {
+  cc_begin();
   constexpr int SLOTS = 4 * CC_SAMPLE;
   __shared__ int s_key[SLOTS], s_cnt[SLOTS];
   __shared__ unsigned long long s_best;
@@ -118,6 +143,7 @@ __global__ void __launch_bounds__(CC_SAMPLE) k_cc_common(const int *comp, int64_
 // end.
 __global__ void __launch_bounds__(CC_THREADS) k_cc_rest(const int64_t *off, const int *col, int64_t n, int *comp,
                                                         cc_state_t *S, cc_piece_t *piece) {
+  cc_begin();
   const int common = S->common, lane = lane_id();
   for (int64_t v0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~int64_t(31); v0 < n;
        v0 += (int64_t)gridDim.x * blockDim.x) {
@@ -147,6 +173,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_rest(const int64_t *off, cons
 }
 __global__ void __launch_bounds__(CC_THREADS) k_cc_pieces(const int *col, int *comp, const cc_state_t *S,
                                                           const cc_piece_t *piece) {
+  cc_begin();
   const int np = S->pieces;
   for (int i = blockIdx.x; i < np; i += gridDim.x) {
     const cc_piece_t p = piece[i];

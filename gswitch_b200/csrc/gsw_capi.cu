@@ -2257,25 +2257,18 @@ static gsw_status cc_forest_run(gsw_ctx *ctx, gsw_graph *gr, int32_t *labels, gs
   if (!comp || !S || !piece) return eg.finish();
   const int grid = clamp_grid((n + CC_THREADS - 1) / CC_THREADS, sm_count() * 8);
   timer tm(ctx);
-  k_cc_start<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp);
-  GSW_LAUNCHED();
   // flat trees before every pass that climbs them (cc_link takes a step at a time)
+  cc_launch(k_cc_start, grid, CC_THREADS, true, gr->off, gr->col, n, comp);
   for (int last = 0; last < 2; ++last) {
-    k_cc_flatten<<<grid, CC_THREADS, 0, stream()>>>(comp, n);
-    GSW_LAUNCHED();
-    k_cc_link_one<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp, last != 0);
-    GSW_LAUNCHED();
+    cc_launch(k_cc_flatten, grid, CC_THREADS, false, comp, n);
+    cc_launch(k_cc_link_one, grid, CC_THREADS, false, gr->off, gr->col, n, comp, last != 0);
   }
-  k_cc_flatten<<<grid, CC_THREADS, 0, stream()>>>(comp, n);
-  GSW_LAUNCHED();
-  k_cc_common<<<1, CC_SAMPLE, 0, stream()>>>(comp, n, S);
-  GSW_LAUNCHED();
-  k_cc_rest<<<grid, CC_THREADS, 0, stream()>>>(gr->off, gr->col, n, comp, S, piece);
-  GSW_LAUNCHED();
-  k_cc_pieces<<<sm_count() * 8, CC_THREADS, 0, stream()>>>(gr->col, comp, S, piece);
-  GSW_LAUNCHED();
-  k_cc_flatten<<<grid, CC_THREADS, 0, stream()>>>(comp, n);
-  GSW_LAUNCHED();
+  cc_launch(k_cc_flatten, grid, CC_THREADS, false, comp, n);
+  cc_launch(k_cc_common, 1, CC_SAMPLE, false, comp, n, S);
+  cc_launch(k_cc_rest, grid, CC_THREADS, false, gr->off, gr->col, n, comp, S, piece);
+  if (gr->max_in_degree < 0 || gr->max_in_degree >= CC_ROW_PIECE)  // rows that may be cut
+    cc_launch(k_cc_pieces, sm_count() * 8, CC_THREADS, false, gr->col, comp, S, piece);
+  cc_launch(k_cc_flatten, grid, CC_THREADS, false, comp, n);
   const double ms = tm.stop();
   if (st) {
     st->ms = ms;

@@ -109,3 +109,19 @@ def test_chains_in_id_order(ctx, case):
     assert all(not lab.any() for lab, _ in runs)  # one component
     assert min(st.ms for _, st in runs) <= 4 * loop + 0.2, (loop, [st.ms for _, st in runs])
     g.close()
+
+
+def test_passes_see_what_the_one_before_wrote(ctx):
+    """The passes are set up while the one before still runs: many runs in a row on
+    graphs of a few and of many CTAs, with other work on the same buffers between."""
+    r = np.random.default_rng(5)
+    for n, m in ((300, 280), (5000, 4000), (200000, 150000), (700000, 600000)):
+        u, v = r.integers(0, n, m), r.integers(0, n, m)
+        off, col = csr(n, np.concatenate([u, v]), np.concatenate([v, u]))
+        g = ctx.upload(off, col)
+        ref = g.cc("x-Bitmap")[0]
+        for k in range(30):
+            assert np.array_equal(g.cc()[0], ref), (n, k)
+            if k % 3 == 0:
+                g.bfs(int(u[k]), out=False)  # takes the labels' buffer for its levels
+        g.close()
