@@ -10,9 +10,15 @@
 // What bounds it is the chain of a level: piece, columns, levels of their
 // vertices, the append and the barrier, about 5 us.  Every level pushes; on
 // larger graphs the pull's early exit saves more than the loop costs.  SB_MAX_*:
-// one call, this against the loop, is 92 against 248 us on RMAT 2^12, 147
-// against 275 on 2^16, 201 against 311 on 2^17 (3.7 M arcs), 281 against 386 on
-// G(2^18, 2^21); RMAT 2^18 has 7.6 M arcs and takes the loop 338 us.
+// one call, this against the loop (timed, its events included), is 73 against 292
+// us on RMAT 2^10, 144 against 384 on 2^16, 198 against 386 on 2^17 (3.7 M arcs),
+// 271 against 412 on 2^18 with 3.9 M arcs, 269 against 360 on G(2^18, 2^21), 177
+// against 235 on a star of 2^18.  Past the line the gain runs out: RMAT 2^18 with
+// 7.6 M arcs 294 against 400, 2^19 with 15.5 M 467 against 487, 2^20 with 31 M 770
+// against 656, G(2^20, 2^21) 949 against 766.  Long graphs keep a level below the
+// loop's persistent one: a lattice of 512 x 512 with 633 levels 3.5 against 5.6 ms,
+// of 64 x 4,096 with 3,902 levels 18.8 against 31.8 ms, a chain of 12,527 levels 43
+// against 84 ms.
 #pragma once
 #include "engine/executor.cuh"
 

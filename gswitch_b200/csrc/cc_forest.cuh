@@ -203,15 +203,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_arc_pairs(const int64_t *off
     }
     __syncwarp();
     for (int e = lane; e < ne; e += 32) {
-      int l = 0, h = cnt;
-      while (l < h) {
-        const int mid = (l + h) >> 1;
-        if (s_beg[mid] <= e)
-          l = mid + 1;
-        else
-          h = mid;
-      }
-      const int v = lo + l - 1, u = ld_stream(col + ea + e);
+      const int v = lo + tile_owner(s_beg, cnt, e), u = ld_stream(col + ea + e);
       if (u > v) {
         ++up;
         balance += sm64(((uint64_t)v << 32) | (unsigned)u);

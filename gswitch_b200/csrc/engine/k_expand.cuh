@@ -1155,6 +1155,20 @@ __global__ void __launch_bounds__(256) k_all_tiles(const int64_t *off, int64_t n
   }
 }
 
+// the vertex of a tile, none before j, that owns the tile's edge r: the last whose
+// edges begin at or before it
+__device__ __forceinline__ int tile_owner(const unsigned short *beg, int cnt, int r, int j = 0) {
+  int l = j, h = cnt;
+  while (l < h) {
+    const int mid = (l + h) >> 1;
+    if (beg[mid] <= r)
+      l = mid + 1;
+    else
+      h = mid;
+  }
+  return l - 1;
+}
+
 template <typename G, typename F>
 __global__ void __launch_bounds__(EXPAND_THREADS, 5) k_pull_all(active_set_t as, G g, F f, config_t conf,
                                                              const int *tile_lo, int64_t ntiles) {
@@ -1209,15 +1223,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS, 5) k_pull_all(active_set_t as,
     int jfirst = -1, j = -1;  // the vertex of the first edge, of the open end
     WA acc = f.data.zero, first = f.data.zero;
     if (a < b) {
-      int l = 0, h = cnt;  // upper bound of a
-      while (l < h) {
-        const int mid = (l + h) >> 1;
-        if (s_beg[mid] <= a)
-          l = mid + 1;
-        else
-          h = mid;
-      }
-      jfirst = j = l - 1;
+      jfirst = j = tile_owner(s_beg, cnt, a);
       int end = s_beg[j + 1];
 #pragma unroll
       for (int k = 0; k < ALL_PER; ++k) {
@@ -1231,15 +1237,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS, 5) k_pull_all(active_set_t as,
           acc = f.data.zero;
           end = s_beg[++j + 1];
           if (r >= end) {  // past vertices without edges, of which a skewed graph has long runs
-            l = j + 1, h = cnt;
-            while (l < h) {
-              const int mid = (l + h) >> 1;
-              if (s_beg[mid] <= r)
-                l = mid + 1;
-              else
-                h = mid;
-            }
-            j = l - 1;
+            j = tile_owner(s_beg, cnt, r, j + 1);
             end = s_beg[j + 1];
           }
         }
@@ -1319,15 +1317,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) k_push_all(active_set_t as, G 
     int j = -1, end = 0;
     for (int r = a; r < b; ++r) {
       if (r >= end) {
-        int l = j + 1, h = cnt;
-        while (l < h) {
-          const int mid = (l + h) >> 1;
-          if (s_beg[mid] <= r)
-            l = mid + 1;
-          else
-            h = mid;
-        }
-        j = l - 1;
+        j = tile_owner(s_beg, cnt, r, j + 1);
         end = s_beg[j + 1];
       }
       s_own[r + lane] = (unsigned short)j;

@@ -56,14 +56,26 @@ def test_matches_the_oracle(ctx, case, directed):
     g.close()
 
 
-@pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1])
-def test_line_to_the_level_loop(ctx, n):
-    r = np.random.default_rng(n)
-    u, v = r.integers(0, n, 200000), r.integers(0, n, 200000)
+@pytest.mark.parametrize("n,m", [((1 << 18) - 1, 400000), (1 << 18, 400000), ((1 << 18) + 1, 400000),
+                                 (1 << 18, (1 << 22) - 2), (1 << 18, 1 << 22), (1 << 18, (1 << 22) + 2),
+                                 (5000, 1 << 22), (5000, (1 << 22) + 2)])
+def test_line_to_the_level_loop(ctx, n, m):
+    """One launch up to 2^18 vertices and 2^22 arcs, the loop from there, with a hub of
+    n - 1 arcs (duplicates too) so that the pieces of one row fill the queues."""
+    r = np.random.default_rng(n + m)
+    u, v = r.integers(0, n, m // 2), r.integers(0, n, m // 2)
+    u[:n // 2] = 7
     off, col = csr(n, np.concatenate([u, v]), np.concatenate([v, u]))
+    assert len(col) == m
     g = ctx.upload(off, col)
-    root = int(u[0])
-    assert np.array_equal(g.bfs(root)[0], oracle.bfs(oracle.Csr(off, col), root))
+    h = oracle.Csr(off, col)
+    for root in (int(v[-1]), 7):
+        lv, st = g.bfs(root)
+        assert np.array_equal(lv, oracle.bfs(h, root))
+        one = n <= 1 << 18 and m <= 1 << 22
+        assert (len(st.trace) == 1 and st.level_persistent == [True]) == one, (len(st.trace), st.level_persistent)
+        loop, ls = g.bfs(root, gs.RunOpts(timing=True))
+        assert np.array_equal(loop, lv) and ls.edges == st.edges
     g.close()
 
 
